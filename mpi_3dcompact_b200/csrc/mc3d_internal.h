@@ -307,11 +307,14 @@ struct MlpDev {
     long long t = 0;                                                 // Adam step
 };
 int mlp_pack(const MlpDev &m, cudaStream_t st);
-int mlp_forward_fp32(const MlpDev &m, const float *x, int n, float *act, float *out, cudaStream_t st);
-// forward, backward and the weight gradients accumulated into m.G (no update)
-int mlp_gradient(MlpDev &m, const float *x, const float *y, int n, float *act, float *out, float *delta,
-                 double *loss, cudaStream_t st);
-int mlp_train_step(MlpDev &m, const float *x, const float *y, int n, float lr, float *act, float *out, float *delta,
+int mlp_forward_fp32(const MlpDev &m, const float *x, int n, float *out, cudaStream_t st);
+// Training workspace: part [MLP_MAXPARTS][MLP_NPARAM], lpart [MLP_MAXPARTS], the
+// gradient and loss sums of the tile kernel's CTAs (at most MLP_MAXPARTS of them).
+constexpr int MLP_MAXPARTS = 256;
+// forward, backward and the weight gradients into m.G (no update)
+int mlp_gradient(MlpDev &m, const float *x, const float *y, int n, float *part, double *lpart, double *loss,
+                 cudaStream_t st);
+int mlp_train_step(MlpDev &m, const float *x, const float *y, int n, float lr, float *part, double *lpart,
                    double *loss, cudaStream_t st);
 // tensor-core inference of raw features x [n][9] -> raw outputs [n][2] (sgs_mlp.cu)
 int mlp_infer_bf16(const MlpDev &m, const float *x, int n, float *out, cudaStream_t st);

@@ -14,25 +14,17 @@ using namespace mc3d;
 struct mc3d_mlp_s {
     MlpDev dev;
     int device = 0;
-    // training workspace, sized for the largest batch seen
-    int cap = 0;
-    float *act = nullptr, *out = nullptr, *delta = nullptr;
+    // training workspace (mlp_gradient), allocated at the first training call
+    float *part = nullptr;
+    double *lpart = nullptr;
     double *loss = nullptr;
 };
 
 namespace {
 
-int mlp_alloc_ws(mc3d_mlp m, int n) {
-    if (n <= m->cap) return MC3D_OK;
-    cudaFree(m->act);
-    cudaFree(m->out);
-    cudaFree(m->delta);
-    m->act = m->out = m->delta = nullptr;
-    m->cap = 0;
-    MC3D_CUDA_TRY(cudaMalloc(&m->act, (size_t)6 * n * 64 * sizeof(float)));
-    MC3D_CUDA_TRY(cudaMalloc(&m->out, (size_t)n * MLP_OUT * sizeof(float)));
-    MC3D_CUDA_TRY(cudaMalloc(&m->delta, ((size_t)3 * n * 64 + (size_t)n * MLP_OUT) * sizeof(float)));
-    m->cap = n;
+int mlp_alloc_ws(mc3d_mlp m) {
+    if (!m->part) MC3D_CUDA_TRY(cudaMalloc(&m->part, (size_t)MLP_MAXPARTS * MLP_NPARAM * sizeof(float)));
+    if (!m->lpart) MC3D_CUDA_TRY(cudaMalloc(&m->lpart, MLP_MAXPARTS * sizeof(double)));
     return MC3D_OK;
 }
 
@@ -97,7 +89,7 @@ int mc3d_mlp_destroy(mc3d_mlp m) {
     if (!m) return MC3D_OK;
     cudaSetDevice(m->device);
     for (void *p : {(void *)m->dev.P, (void *)m->dev.G, (void *)m->dev.M, (void *)m->dev.V, (void *)m->dev.Tw,
-                    (void *)m->act, (void *)m->out, (void *)m->delta, (void *)m->loss})
+                    (void *)m->part, (void *)m->lpart, (void *)m->loss})
         if (p) cudaFree(p);
     delete m;
     return MC3D_OK;
@@ -139,11 +131,10 @@ int mc3d_mlp_get_normalization(mc3d_mlp m, float *out /* 4*9 + 2*2 */) {
 int mc3d_mlp_train_step(mc3d_mlp m, const float *x, const float *y, int n, float lr, double *loss, void *stream) {
     if (!m || !x || !y || n <= 0) return fail(MC3D_ERR_ARG, "bad argument");
     MC3D_CUDA_TRY(cudaSetDevice(m->device));
-    int rc = mlp_alloc_ws(m, n);
+    int rc = mlp_alloc_ws(m);
     if (rc) return rc;
     cudaStream_t st = (cudaStream_t)stream;
-    MC3D_CUDA_TRY(cudaMemsetAsync(m->loss, 0, sizeof(double), st));
-    if ((rc = mlp_train_step(m->dev, x, y, n, lr, m->act, m->out, m->delta, m->loss, st))) return rc;
+    if ((rc = mlp_train_step(m->dev, x, y, n, lr, m->part, m->lpart, m->loss, st))) return rc;
     if (loss) {
         MC3D_CUDA_TRY(cudaMemcpyAsync(loss, m->loss, sizeof(double), cudaMemcpyDeviceToHost, st));
         MC3D_CUDA_TRY(cudaStreamSynchronize(st));
@@ -154,16 +145,12 @@ int mc3d_mlp_train_step(mc3d_mlp m, const float *x, const float *y, int n, float
 int mc3d_mlp_gradient(mc3d_mlp m, const float *x, const float *y, int n, float *G, double *loss, void *stream) {
     if (!m || !x || !y || !G || n <= 0) return fail(MC3D_ERR_ARG, "bad argument");
     MC3D_CUDA_TRY(cudaSetDevice(m->device));
-    int rc = mlp_alloc_ws(m, n);
+    int rc = mlp_alloc_ws(m);
     if (rc) return rc;
     cudaStream_t st = (cudaStream_t)stream;
-    MC3D_CUDA_TRY(cudaMemsetAsync(m->loss, 0, sizeof(double), st));
-    MC3D_CUDA_TRY(cudaMemsetAsync(m->dev.G, 0, MLP_NPARAM * sizeof(float), st));
-    if ((rc = mlp_gradient(m->dev, x, y, n, m->act, m->out, m->delta, m->loss, st))) return rc;
+    if ((rc = mlp_gradient(m->dev, x, y, n, m->part, m->lpart, m->loss, st))) return rc;
     MC3D_CUDA_TRY(cudaMemcpyAsync(G, m->dev.G, MLP_NPARAM * sizeof(float), cudaMemcpyDeviceToHost, st));
     if (loss) MC3D_CUDA_TRY(cudaMemcpyAsync(loss, m->loss, sizeof(double), cudaMemcpyDeviceToHost, st));
-    // the training step expects a zero gradient buffer
-    MC3D_CUDA_TRY(cudaMemsetAsync(m->dev.G, 0, MLP_NPARAM * sizeof(float), st));
     MC3D_CUDA_TRY(cudaStreamSynchronize(st));
     return MC3D_OK;
 }
@@ -171,7 +158,7 @@ int mc3d_mlp_gradient(mc3d_mlp m, const float *x, const float *y, int n, float *
 int mc3d_mlp_forward(mc3d_mlp m, const float *x, float *y, int n, void *stream) {
     if (!m || !x || !y || n <= 0) return fail(MC3D_ERR_ARG, "bad argument");
     MC3D_CUDA_TRY(cudaSetDevice(m->device));
-    return mlp_forward_fp32(m->dev, x, n, nullptr, y, (cudaStream_t)stream);
+    return mlp_forward_fp32(m->dev, x, n, y, (cudaStream_t)stream);
 }
 
 int mc3d_mlp_infer_bf16(mc3d_mlp m, const float *x, float *y, int n, void *stream) {

@@ -43,9 +43,11 @@ constexpr float GELU_K0 = 0.7978845608028654f, GELU_K1 = 0.044715f;
 __device__ __forceinline__ float gelu(float x) {
     return 0.5f * x * (1.0f + tanhf(GELU_K0 * (x + GELU_K1 * x * x * x)));
 }
-__device__ __forceinline__ float gelu_grad(float x) {
+// and its derivative, from the same tanh
+__device__ __forceinline__ void gelu_both(float x, float &h, float &g) {
     const float t = tanhf(GELU_K0 * (x + GELU_K1 * x * x * x));
-    return 0.5f * (1.0f + t) + 0.5f * x * (1.0f - t * t) * GELU_K0 * (1.0f + 3.0f * GELU_K1 * x * x);
+    h = 0.5f * x * (1.0f + t);
+    g = 0.5f * (1.0f + t) + 0.5f * x * (1.0f - t * t) * GELU_K0 * (1.0f + 3.0f * GELU_K1 * x * x);
 }
 // two FP32 values as a BF16 pair (lo in the low half), round to nearest even
 __device__ __forceinline__ unsigned pack_bf2(float lo, float hi) {

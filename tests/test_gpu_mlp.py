@@ -138,6 +138,31 @@ def test_gradient_matches_numpy_by_value():
     assert np.array_equal(mlp.params(), P)
 
 
+@pytest.mark.parametrize("n", [1, 127, 129, 19001])
+def test_gradient_of_ragged_batches(n):
+    """Batches that end inside a tile of 128 samples, below one tile and above
+    one tile per CTA (148 x 128 = 18944), against the float64 gradient: relative
+    L2 per parameter block as in the test above, the FP32 sums being no longer
+    than there (at most two tiles a CTA, then 148 CTAs)."""
+    torch = _torch()
+    mlp, P, mean, std, rng = _mlp_with_random_params(6)
+    x = rng.standard_normal((n, 9)).astype(np.float32)
+    y = rng.standard_normal((n, 2)).astype(np.float32)
+    xt, yt = torch.tensor(x, device="cuda"), torch.tensor(y, device="cuda")
+    G, loss = mlp.gradient(xt, yt)
+    ref = np_grad(P.astype(np.float64), x.astype(np.float64), y.astype(np.float64), mean.astype(np.float64),
+                  std.astype(np.float64))
+    _, out = np_forward(P.astype(np.float64), x.astype(np.float64), mean.astype(np.float64), std.astype(np.float64))
+    assert abs(loss - np.mean(np.sum((out - y) ** 2, axis=1))) <= 1e-5 * loss
+    bounds = sorted(OFF.values()) + [9090]
+    for a, b in zip(bounds[:-1], bounds[1:]):
+        g, r = G[a:b].astype(np.float64), ref[a:b]
+        assert np.linalg.norm(g - r) <= 2e-5 * np.linalg.norm(r), (a, b)
+    yf = torch.empty((n, 2), dtype=torch.float32, device="cuda")
+    mlp.forward(xt, yf)
+    assert np.abs(yf.cpu().numpy() - out).max() <= 1e-5 * np.abs(out).max()
+
+
 def test_adam_first_step_follows_the_gradient():
     torch = _torch()
     mlp, P, mean, std, rng = _mlp_with_random_params(3)
