@@ -490,38 +490,56 @@ void analyse(LineOpHost &h, int precision) {
     }
 }
 
+// Is the interior stencil of h antisymmetric with a zero centre (the first
+// derivatives), so that a row's RHS is sum_k st[H+k] (phi[n+k] - phi[n-k])?
+bool antisymmetric(const LineOpHost &h) {
+    if (h.H < 1 || h.H > 3 || h.st[h.H] != 0.0) return false;
+    for (int k = 1; k <= h.H; k++)
+        if (h.st[h.H + k] != -h.st[h.H - k]) return false;
+    for (int k = 2 * h.H + 1; k < 11; k++)
+        if (h.st[k] != 0.0) return false;
+    return true;
+}
+
 // Segment count and homogeneous responses for the segmented line solve.
 // tri:   forward  x_n = -m_n x_{n-1}                        from x_{a-1} = 1
 //        backward x_n = -c_n x_{n+1} rw_n                    from x_b = 1
 // penta: forward  B_n = -m2_{n-1} B_{n-2} - m1_n B_{n-1}     from (B_{a-1}, B_{a-2}) = (1,0) | (0,1)
 //        backward x_n = (-f_n x_{n+2} - C_n x_{n+1}) rD_n    from (x_b, x_{b+1}) = (1,0) | (0,1)
-void segment(LineOpHost &h, int precision) {
+void segment(LineOpHost &h, int precision, bool ragged) {
     int n = h.N;
     bool tri = h.kind == K_TRI_PER || h.kind == K_TRI_DIR;
     bool pen = h.kind == K_PEN_PER || h.kind == K_PEN_DIR;
     h.S = 1;
     h.L = 0;
+    h.rag = false;
     if (!(tri || pen)) return;
     const int UB = 8;
     int S = 0;
     int Lr = reg_segment_len(n, h.kind, precision);
+    int L = 0;
     if (Lr) {
         S = n / Lr;
         h.L = Lr;
+    } else if (int Lg = ragged && !(precision != MC3D_FP64 && h.H <= 3 && !antisymmetric(h))
+                            ? ragged_segment_len(n, h.kind) : 0) {   // (the FP32 solve of H <= 3: derivatives only)
+        h.L = L = Lg;
+        h.rag = true;
+        S = (n + L - 1) / L;
     } else {
         for (int cand : {4, 2})
             if (n % cand == 0 && (n / cand) % UB == 0 && n / cand >= 32 && n / cand >= h.bw) { S = cand; break; }
     }
     if (!S) return;
     h.S = S;
-    int L = n / S;
+    if (!L) L = n / S;
     auto A = [&](int a, int i) { return h.arr[(size_t)a * n + i]; };
     h.sfa.assign(n, 0.0);
     h.sfb.assign(n, 0.0);
     h.sba.assign(n, 0.0);
     h.sbb.assign(n, 0.0);
     for (int w = 0; w < S; w++) {
-        int a = w * L, b = a + L;
+        int a = w * L, b = std::min(a + L, n);
         for (int which = 0; which < (pen ? 2 : 1); which++) {
             // forward
             double p1 = which == 0 ? 1.0 : 0.0, p2 = which == 0 ? 0.0 : 1.0;   // B_{n-1}, B_{n-2}
@@ -552,17 +570,6 @@ struct Layout {
     size_t arr = 0, head = 0, tail = 0, seg = 0;
     size_t pf = 0, pb = 0, pz = 0, sf2 = 0, sb2 = 0, hp = 0, tp = 0, pbs = 0;
 };
-
-// Is the interior stencil of h antisymmetric with a zero centre (the first
-// derivatives), so that a row's RHS is sum_k st[H+k] (phi[n+k] - phi[n-k])?
-bool antisymmetric(const LineOpHost &h) {
-    if (h.H < 1 || h.H > 3 || h.st[h.H] != 0.0) return false;
-    for (int k = 1; k <= h.H; k++)
-        if (h.st[h.H + k] != -h.st[h.H - k]) return false;
-    for (int k = 2 * h.H + 1; k < 11; k++)
-        if (h.st[k] != 0.0) return false;
-    return true;
-}
 
 template <typename R>
 void fill_dev(const LineOpHost &h, const char *base, const Layout &lo, LineOpDev<R> &d) {
@@ -606,7 +613,7 @@ void fill_dev(const LineOpHost &h, const char *base, const Layout &lo, LineOpDev
     d.head = h.head.empty() ? nullptr : p + lo.head;
     d.tail = h.tail.empty() ? nullptr : p + lo.tail;
     const R *sg = p + lo.seg;
-    d.S = h.S;
+    d.S = h.rag ? 1 : h.S;   // (the shared-memory kernels take equal segments only)
     d.seg_kf = h.seg_kf;
     d.seg_kb = h.seg_kb;
     d.sfa = h.S > 1 ? sg : nullptr;
@@ -614,6 +621,7 @@ void fill_dev(const LineOpHost &h, const char *base, const Layout &lo, LineOpDev
     d.sba = h.S > 1 ? sg + 2 * n : nullptr;
     d.sbb = h.S > 1 ? sg + 3 * n : nullptr;
     d.L = h.L;
+    d.rag = h.rag;
     d.pf = h.L ? p + lo.pf : nullptr;
     d.pb = h.L ? p + lo.pb : nullptr;
     d.pz = h.L && h.kind == K_PEN_PER ? p + lo.pz : nullptr;
@@ -646,12 +654,17 @@ std::vector<R> flatten(const LineOpHost &h, Layout &lo) {
         const int n = h.N;
         const bool tri = h.kind == K_TRI_PER || h.kind == K_TRI_DIR;
         auto A = [&](int a, int i) { return h.arr[(size_t)a * n + i]; };
+        // zero rows past the end fill the last segment (and two rows more, read by the chains)
+        auto pad = [&](int width) {
+            for (int i = 0; h.rag && i < ((n + h.L - 1) / h.L * h.L - n + 2) * width; i++) put(0.0);
+        };
         align4();
         lo.pf = v.size();
         for (int i = 0; i < n; i++) {
             put(i >= 1 ? A(0, i) : 0.0);
             put(!tri && i >= 2 ? A(1, i - 1) : 0.0);
         }
+        pad(2);
         align4();
         lo.pb = v.size();
         for (int i = 0; i < n; i++) {
@@ -666,6 +679,7 @@ std::vector<R> flatten(const LineOpHost &h, Layout &lo) {
             }
             put(0.0);
         }
+        pad(4);
         align4();
         lo.pbs = v.size();
         for (int i = 0; i < n; i++) {
@@ -675,11 +689,13 @@ std::vector<R> flatten(const LineOpHost &h, Layout &lo) {
             put(rD);
             put(0.0);
         }
+        pad(4);
         if (h.kind == K_PEN_PER) {
             align4();
             lo.pz = v.size();
             for (int i = 0; i < n; i++)
                 for (int c = 0; c < 4; c++) put(A(5 + c, i));
+            pad(4);
         }
         align4();
         lo.sf2 = v.size();
@@ -693,6 +709,7 @@ std::vector<R> flatten(const LineOpHost &h, Layout &lo) {
             put(h.sba[i]);
             put(h.sbb[i]);
         }
+        pad(2);
         if (h.kind == K_TRI_DIR || h.kind == K_PEN_DIR) {
             const int bw = h.bw, B = MC3D_BWMAX;
             lo.hp = v.size();
@@ -718,20 +735,28 @@ int reg_segment_len(int N, int kind, int precision) {
     return 0;
 }
 
-int upload_line_op(const LineOpHost &hin, int precision, LineOpBuf &out) {
+int ragged_segment_len(int N, int kind) {
+    if (!(kind == K_TRI_PER || kind == K_TRI_DIR || kind == K_PEN_PER || kind == K_PEN_DIR)) return 0;
+    // a boundary row must fit the line, and 16 warps of 32 rows hold 512
+    if (N < MC3D_BWMAX || N > 16 * 32) return 0;
+    return 32;
+}
+
+int upload_line_op(const LineOpHost &hin, int precision, LineOpBuf &out, bool ragged) {
     LineOpHost h = hin;
     if (h.bw > MC3D_BWMAX) return fail(MC3D_ERR_CONFIG, "boundary row wider than the kernels support");
     analyse(h, precision);
-    segment(h, precision);
+    segment(h, precision, ragged);
     if (h.S > 1) {
         // responses below 2^-64 (FP64) / 2^-32 (FP32) of their unit start are dropped
         const double thr = std::ldexp(1.0, precision == MC3D_FP64 ? -64 : -32);
-        int n = h.N, L = n / h.S;
+        int n = h.N, L = h.rag ? h.L : n / h.S;
         h.seg_kf = h.seg_kb = 0;
         for (int w = 0; w < h.S; w++)
-            for (int r = 0; r < L; r++) {
+            for (int r = 0; r < L && w * L + r < n; r++) {
                 int i = w * L + r;
                 if (std::fabs(h.sfa[i]) > thr || std::fabs(h.sfb[i]) > thr) h.seg_kf = std::max(h.seg_kf, r + 1);
+                if (h.rag && w == h.S - 1) continue;   // (nothing comes back into the last segment)
                 if (std::fabs(h.sba[i]) > thr || std::fabs(h.sbb[i]) > thr) h.seg_kb = std::max(h.seg_kb, L - r);
             }
     }

@@ -103,11 +103,15 @@ struct LineOpHost {
     // backward responses are above the precision's cut-off (set at upload)
     int seg_kf = 0, seg_kb = 0;
     int L = 0;   // segment length of the register-resident kernel (0: not used)
+    bool rag = false;   // N is no multiple of L: the last segment has fewer rows
 };
 
 // Segment length of the register-resident line solve for a line of N points
 // in a precision (0 when the line goes to the shared-memory kernels).
 int reg_segment_len(int N, int kind, int precision);
+// The same for the other lengths, the last segment having fewer rows (0 when the
+// line goes to the shared-memory kernels).
+int ragged_segment_len(int N, int kind);
 
 LineOpHost build_deriv_op(int fd_type, int bc_type, int N, double dh);
 LineOpHost build_filter_op(int filter_type, double alphaF, int bc_type, int N);
@@ -145,6 +149,7 @@ struct LineOpDev {
     //   hp, tp [H][MC3D_BWMAX]  Dirichlet boundary rows, zero padded (head on
     //   phi[0..BWMAX-1], tail right-aligned on phi[N-BWMAX..N-1])
     int L;
+    int rag;   // N is no multiple of L: the last of ceil(N / L) segments has fewer rows
     const R *pf, *pb, *pz, *sf2, *sb2, *hp, *tp;
     // FP32 derivative form of the register-resident solve (H <= 3): asym is 1
     // when the interior stencil is antisymmetric with a zero centre, sta[k-1]
@@ -166,7 +171,9 @@ struct LineOpBuf {
     int precision = MC3D_FP64;
     int device = 0;
 };
-int upload_line_op(const LineOpHost &h, int precision, LineOpBuf &out);
+// ragged: lines that are no multiple of the segment length may be solved in
+// segments, whose superposition sums in another order than the whole-line solve
+int upload_line_op(const LineOpHost &h, int precision, LineOpBuf &out, bool ragged = true);
 void free_line_op(LineOpBuf &b);
 
 // ---- sweep launch ---------------------------------------------------------

@@ -103,6 +103,15 @@ struct mc3d_solver_s {
 
 namespace mc3d {
 
+// Whether a solver's lines may take the ragged segmented solve. Not with the
+// dynamic model in FP32: its coefficient is a ratio of averages that magnifies
+// the operators' rounding (another order of the same FP32 sums moves the
+// spanwise momentum of an O-grid by 2e-5 relative within two steps, the distance
+// of either from FP64 being 4e-5), so those solvers keep the whole-line order.
+static bool ragged_lines(int les_model, int precision) {
+    return !(les_model == MC3D_DSM && precision != MC3D_FP64);
+}
+
 // FP64 partial sums of GLOBAL averaging: up to 148 x 4 blocks for up to 8 fields
 constexpr size_t AVG_SCRATCH = 148 * 4 * 8;
 
@@ -977,14 +986,14 @@ int mc3d_solver_create(const mc3d_config *cfg, int device, mc3d_solver *out) {
             LineOpHost dh = build_deriv_op(c.fd_type[d], c.bc_type[d], N[d], s->dxi[d]);
             LineOpHost fh = build_filter_op(c.filter_type, c.alphaF, c.bc_type[d], N[d]);
             LineOpHost vh = build_filter_op(MC3D_COMPACT10, -0.49, c.bc_type[d], N[d]);
-            if ((rc = upload_line_op(dh, c.precision, s->dop[d]))) break;
-            if ((rc = upload_line_op(fh, c.precision, s->fop[d]))) break;
-            if ((rc = upload_line_op(vh, c.precision, s->vop[d]))) break;
+            if ((rc = upload_line_op(dh, c.precision, s->dop[d], ragged_lines(c.les_model, c.precision)))) break;
+            if ((rc = upload_line_op(fh, c.precision, s->fop[d], ragged_lines(c.les_model, c.precision)))) break;
+            if ((rc = upload_line_op(vh, c.precision, s->vop[d], ragged_lines(c.les_model, c.precision)))) break;
             if (c.les_model == MC3D_DSM || c.les_model == MC3D_MLPSGS) {
                 // DSMTESTFILTER 1 -> Pade, 2 -> explicit (src/DSMSGS.hpp:57-67)
                 LineOpHost th = build_testfilter_op(c.dsm_test_filter == 1 ? MC3D_TESTFILTER_PADE : MC3D_TESTFILTER_EXP,
                                                     c.bc_type[d], N[d]);
-                if ((rc = upload_line_op(th, c.precision, s->top[d]))) break;
+                if ((rc = upload_line_op(th, c.precision, s->top[d], ragged_lines(c.les_model, c.precision)))) break;
             }
         }
     } catch (const std::exception &ex) {
@@ -1275,7 +1284,7 @@ static int compute_metrics(mc3d_solver s, const double *hx, const double *hy, co
     try {
         for (int d = 0; d < 3 && !rc; d++) {
             LineOpHost h = build_deriv_op(s->cfg.fd_type[d], s->cfg.bc_type[d], Ns[d], s->dxi[d]);
-            if ((rc = upload_line_op(h, MC3D_FP64, md[d].deriv))) break;
+            if ((rc = upload_line_op(h, MC3D_FP64, md[d].deriv, ragged_lines(s->cfg.les_model, s->prec)))) break;
             md[d].periodic = s->cfg.bc_type[d] == MC3D_PERIODIC_SOLVE;
             md[d].cd2 = s->cfg.fd_type[d] == MC3D_CD2;
             md[d].H = h.H;
@@ -1287,7 +1296,7 @@ static int compute_metrics(mc3d_solver s, const double *hx, const double *hy, co
                 sv.st[sv.H] = 1.0;
                 sv.deriv = false;
                 sv.inv_dh = 1.0;
-                rc = upload_line_op(sv, MC3D_FP64, md[d].solve);
+                rc = upload_line_op(sv, MC3D_FP64, md[d].solve, ragged_lines(s->cfg.les_model, s->prec));
             }
         }
     } catch (const std::exception &e) {

@@ -100,6 +100,11 @@ template <int DIR, typename R>
 int launch_sweep_reg(const Grid3 &g, const LineOpDev<R> &op, const SweepBatch<R> &b, int epi,
                      const RhsFinalArgs<R> &rf, int px, int py, int pz, cudaStream_t st);
 
+// The same for line lengths that are no multiple of the segment length.
+template <int DIR, typename R>
+int launch_sweep_rag(const Grid3 &g, const LineOpDev<R> &op, const SweepBatch<R> &b, int epi,
+                     const RhsFinalArgs<R> &rf, int px, int py, int pz, cudaStream_t st);
+
 // FP32 x-line solves staged through shared memory by TMA (sweep_tma.cuh,
 // sweeps_tma.cu);
 // MC3D_ERR_CONFIG, without recording an error, when the case is not covered

@@ -70,9 +70,10 @@ struct RegVec<double> {
 // block of UB rows ahead of the block being stored, in program order before
 // those stores, so each block costs one memory round trip at most and the
 // loads overlap the previous block's stores.
-template <typename R, int E, int L, bool PREFETCH = true>
+// RAG: only the segment's first Lw rows exist.
+template <typename R, int E, int L, bool PREFETCH = true, bool RAG = false>
 __device__ __forceinline__ void reg_store_rows(const SweepBatch<R> &b, const RhsFinalArgs<R> &rf, int f, int off0,
-                                               int stride, const R (&y)[L]) {
+                                               int stride, const R (&y)[L], int Lw = L) {
     constexpr int NB = L / UB;
     constexpr bool RD_OLD = E == EPI_SUB || E == EPI_RHS_FINAL;   // RHS_FINAL: only momentum with the quirk
     constexpr bool RD_AUX = E == EPI_RHS_FINAL;
@@ -91,6 +92,7 @@ __device__ __forceinline__ void reg_store_rows(const SweepBatch<R> &b, const Rhs
     auto fetch = [&](int blk, int slot) {
 #pragma unroll
         for (int u = 0; u < UB; u++) {
+            if (RAG && blk * UB + u >= Lw) break;
             const int off = off0 + (blk * UB + u) * stride;
             if (RD_OLD) old[slot][u] = rd_old ? o[off] : R(0);
             if (RD_AUX) {
@@ -108,6 +110,7 @@ __device__ __forceinline__ void reg_store_rows(const SweepBatch<R> &b, const Rhs
 #pragma unroll
         for (int u = 0; u < UB; u++) {
             const int r = blk * UB + u;
+            if (RAG && r >= Lw) break;
             const int off = off0 + r * stride;
             const R v = y[r];
             if (E == EPI_STORE) o[off] = v;
@@ -186,6 +189,59 @@ __device__ __forceinline__ void reg_copy_out(const SweepBatch<R> &b, const RhsFi
     }
 }
 
+// x lines of any length: the tile's nl lines go round the S warps, each line's
+// values round the lanes (whole lines, so that rows of any length stay
+// contiguous across the warp); the read operands of four groups of 32 values
+// are loaded before the groups' stores.
+template <typename R, int E>
+__device__ __forceinline__ void rag_copy_out(const SweepBatch<R> &b, const RhsFinalArgs<R> &rf, int f, int tile0,
+                                             int N, int nl, int seg, int S, int lane, const R *tile) {
+    constexpr int P = W + 1;
+    constexpr int G = 4;
+    constexpr bool RD_OLD = E == EPI_SUB || E == EPI_RHS_FINAL;
+    constexpr bool RD_AUX = E == EPI_RHS_FINAL;
+    const R dt = (E == EPI_RHS_FINAL) ? (R)(*rf.dt) : R(0);
+    const bool mom = (E == EPI_RHS_FINAL) && rf.quirk && b.eq[f] >= 1 && b.eq[f] <= 3;
+    const bool rd_old = E == EPI_SUB || mom;
+    R *o = b.out[f];
+    double *o64 = b.out64[f];
+    const R *ax = b.aux[f];
+    const R *jp = rf.J;
+    for (int l = seg; l < nl; l += S) {
+        const int line0 = (tile0 + l) * N;
+        for (int i0 = 0; i0 < N; i0 += 32 * G) {
+            R old[G], aux[G], jj[G];
+#pragma unroll
+            for (int q = 0; q < G; q++) {
+                const int i = i0 + 32 * q + lane;
+                if (i < N) {
+                    if (RD_OLD) old[q] = rd_old ? o[line0 + i] : R(0);
+                    if (RD_AUX) {
+                        aux[q] = ax[line0 + i];
+                        jj[q] = jp ? jp[line0 + i] : rf.Jc;
+                    }
+                }
+            }
+#pragma unroll
+            for (int q = 0; q < G; q++) {
+                const int i = i0 + 32 * q + lane;
+                if (i >= N) break;
+                const int off = line0 + i;
+                const R v = tile[i * P + l];
+                if (E == EPI_STORE) o[off] = v;
+                if (E == EPI_STORE_NEG) o[off] = -v;
+                if (E == EPI_SUB) o[off] = old[q] - v;
+                if (E == EPI_STORE_F64) o64[off] = (double)v;
+                if (E == EPI_RHS_FINAL) {
+                    R tt = aux[q] - v;
+                    R dtJ = dt * jj[q];
+                    o[off] = mom ? (old[q] + tt) * dtJ : tt * dtJ;
+                }
+            }
+        }
+    }
+}
+
 // E: the caller's operation (EpiMode), compiled into the kernel so that each
 // instantiation carries one epilogue only.
 // The solve of one tile once each lane holds rows a-H .. a+L+H-1 of its line
@@ -204,9 +260,21 @@ __device__ __forceinline__ void reg_copy_out(const SweepBatch<R> &b, const RhsFi
 struct NoFwdHook {
     __device__ __forceinline__ void operator()(int) const {}
 };
-template <typename R, int KIND, int H, int L, bool NEG = false, typename FwdHook = NoFwdHook>
+//
+// RAG: line lengths that are no multiple of L; the last segment has fewer rows.
+// Rows past the line's end are rows of zeros (zero right-hand side, zero
+// factors: the factor arrays are padded to whole segments), which leave the
+// recurrences' zero start values as they are, so every warp runs the same
+// code. tail_at(k) is the line's value N - BWMAX + k (the Dirichlet rows at the
+// end may need more rows than the last segment has).
+struct NoTail {
+    __device__ __forceinline__ float operator()(int) const { return 0.0f; }
+};
+template <typename R, int KIND, int H, int L, bool NEG = false, typename FwdHook = NoFwdHook, bool RAG = false,
+          typename Tail = NoTail>
 __device__ __forceinline__ void reg_solve(const LineOpDev<R> &op, const R (&v)[L + 2 * H], R (&y)[L], bool work,
-                                          int lane, int seg, int S, int a, R *sh, const FwdHook &hook = FwdHook()) {
+                                          int lane, int seg, int S, int a, R *sh, const FwdHook &hook = FwdHook(),
+                                          const Tail &tail_at = Tail()) {
     constexpr bool PER = (KIND % 2) == 0;
     constexpr bool TRI = KIND == K_TRI_PER || KIND == K_TRI_DIR;
     constexpr int NB = L / UB;
@@ -236,7 +304,12 @@ __device__ __forceinline__ void reg_solve(const LineOpDev<R> &op, const R (&v)[L
 #pragma unroll
                 for (int k = 0; k < MC3D_BWMAX; k++) hs += ldc(op.hp + r * MC3D_BWMAX + k) * v[H + k];
             }
-            if (seg == S - 1) {
+            if constexpr (RAG) {
+                if (a + L > N - H) {
+#pragma unroll
+                    for (int k = 0; k < MC3D_BWMAX; k++) ts += ldc(op.tp + r * MC3D_BWMAX + k) * tail_at(k);
+                }
+            } else if (seg == S - 1) {
 #pragma unroll
                 for (int k = 0; k < MC3D_BWMAX; k++) ts += ldc(op.tp + r * MC3D_BWMAX + k) * v[H + L - MC3D_BWMAX + k];
             }
@@ -294,6 +367,7 @@ __device__ __forceinline__ void reg_solve(const LineOpDev<R> &op, const R (&v)[L
                         if (n == N - 1 - q) rr = tailr[q];
                     }
                 }
+                if (RAG && n >= N) rr = R(0);
                 R m1, m2;
                 V::ld2(op.pf + 2 * n, m1, m2);
                 R x = TRI ? rr - m1 * y1 : rr - m2 * y2 - m1 * y1;
@@ -419,7 +493,15 @@ __device__ __forceinline__ void reg_solve(const LineOpDev<R> &op, const R (&v)[L
     }
     bwdStart[(seg * 2 + 0) * W + lane] = y[0];
     bwdStart[(seg * 2 + 1) * W + lane] = y[1];
-    if (seg == S - 1) {
+    if constexpr (RAG) {
+        if (PER && a + L >= N - 1) {
+#pragma unroll
+            for (int r = 0; r < L; r++) {
+                if (a + r == N - 1) lastx[lane] = y[r];
+                if (a + r == N - 2) lastx[W + lane] = y[r];
+            }
+        }
+    } else if (seg == S - 1) {
         lastx[lane] = y[L - 1];
         lastx[W + lane] = y[L - 2];
     }
@@ -454,6 +536,9 @@ __device__ __forceinline__ void reg_solve(const LineOpDev<R> &op, const R (&v)[L
             R x0 = bwdStart[0 * W + lane] + b0a * Y1 + b0b * Y2;
             R x1 = bwdStart[1 * W + lane] + b1a * Y1 + b1b * Y2;
             R xN1 = lastx[lane], xN2 = lastx[W + lane];
+            // a last segment of one row: x_{N-2} ends the segment before it
+            // and still lacks that segment's response to x_{N-1}
+            if (RAG && S > 1 && (S - 1) * L == N - 1) xN2 += ldc(op.sb2 + 2 * (N - 2)) * xN1;
             if (KIND == K_TRI_PER) {
                 // Sherman-Morrison factor (src/Utils.cpp:43)
                 c[0] = (x0 + op.sc[0] * xN1 * op.sc[1]) * op.sc[2];
@@ -522,6 +607,7 @@ __device__ __forceinline__ void reg_solve(const LineOpDev<R> &op, const R (&v)[L
 #pragma unroll
                 for (int u = 0; u < UB; u++) {
                     const int n = n0 + u;
+                    if (RAG && n >= N) break;
                     if (KIND == K_TRI_PER) {
                         y[blk * UB + u] -= c0 * ldc(op.a3 + n);
                     } else {
@@ -630,12 +716,103 @@ __global__ void __launch_bounds__(512) sweep_reg_kernel(Grid3 g, LineOpDev<R> op
     }
 }
 
+// Lines whose length is no multiple of the segment length (the RAG form of
+// reg_solve): S = ceil(N / L) warps, the last with the rows that are left.
+// Bound by the latency of the recurrences, like the other line solves; the
+// whole-line kernel that served these lengths before (one warp a tile, every
+// recurrence over all N rows, each row through shared memory) kept 8 warps an
+// SM busy where this keeps 16.
 template <int DIR, typename R, int KIND, int H, int L, int E>
+__global__ void __launch_bounds__(512) sweep_rag_kernel(Grid3 g, LineOpDev<R> op, SweepBatch<R> b,
+                                                        RhsFinalArgs<R> rf, int pass_y, int pass_z, int pass_x) {
+    constexpr bool PER = (KIND % 2) == 0;
+    constexpr int NV = L + 2 * H;
+    constexpr int P = W + 1;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    R *sh = reinterpret_cast<R *>(smem_raw);
+    const int S = blockDim.x >> 5;
+    const int lane = threadIdx.x & 31, seg = threadIdx.x >> 5;
+    const int N = op.N, a = seg * L;
+    const int Lw = N - a < L ? N - a : L;
+    const int f = blockIdx.y;
+    R *tile = sh + reg_chain_elems(S);   // x lines: [N][W+1], after the chain states
+
+    const TileGeom t = tile_geom<DIR>(g, blockIdx.x, lane);
+    bool pass = false;
+    if (DIR == 0) pass = (pass_y && (t.j == 0 || t.j == g.Ny - 1)) || (pass_z && (t.k == 0 || t.k == g.Nz - 1));
+    if (DIR == 1) pass = (pass_x && (t.i == 0 || t.i == g.Nx - 1)) || (pass_z && (t.k == 0 || t.k == g.Nz - 1));
+    if (DIR == 2) pass = (pass_y && (t.j == 0 || t.j == g.Ny - 1)) || (pass_x && (t.i == 0 || t.i == g.Nx - 1));
+    const bool work = t.active && !pass;
+
+    // ---- load rows a-H .. a+L+H-1 of this lane's line (periodic wrap / zero) ----
+    int nl = W;
+    const R *src;
+    if (DIR == 0) {
+        const long long rem = (long long)g.Ny * g.Nz - (long long)blockIdx.x * W;
+        nl = rem < W ? (int)rem : W;
+        src = b.in[f] + (size_t)blockIdx.x * W * N;
+        // the lines go round the warps, each line's values round the lanes
+        for (int l = seg; l < nl; l += S)
+            for (int i = lane; i < N; i += 32) cp_async_elem(&tile[i * P + l], src + l * N + i);
+        cp_async_wait_all();
+        __syncthreads();
+    } else {
+        src = b.in[f] + (int)t.base;
+    }
+    const int stride = (int)t.stride;
+    auto row = [&](int n) -> R {
+        if (DIR == 0) return tile[n * P + lane];
+        return t.active ? src[n * stride] : R(0);
+    };
+    R v[NV];
+    if (a >= H && a + L + H <= N) {
+#pragma unroll
+        for (int k = 0; k < NV; k++) v[k] = row(a - H + k);
+    } else {
+#pragma unroll
+        for (int k = 0; k < NV; k++) {
+            int n = a - H + k;
+            bool in = true;
+            if (n < 0) {
+                n += N;
+                in = PER;
+            } else if (n >= N) {
+                n -= N;
+                in = PER && n < H;
+            }
+            v[k] = in ? row(n) : R(0);
+        }
+    }
+
+    R y[L];
+    reg_solve<R, KIND, H, L, false, NoFwdHook, true>(op, v, y, work, lane, seg, S, a, sh, NoFwdHook(),
+                                                     [&](int k) { return row(N - MC3D_BWMAX + k); });
+
+    // ---- epilogue ----
+    if (DIR == 0) {
+        // (every lane's line values were read before the solve's barriers)
+        if (t.active) {
+#pragma unroll
+            for (int r = 0; r < L; r++)
+                if (r < Lw) tile[(a + r) * P + lane] = y[r];
+        }
+        __syncthreads();
+        rag_copy_out<R, E>(b, rf, f, (int)blockIdx.x * W, N, nl, seg, S, lane, tile);
+    } else if (t.active) {
+        const int off0 = (int)t.base + a * stride;
+        if (Lw == L) reg_store_rows<R, E, L>(b, rf, f, off0, stride, y);
+        else reg_store_rows<R, E, L, true, true>(b, rf, f, off0, stride, y, Lw);
+    }
+}
+
+template <int DIR, typename R, int KIND, int H, int L, int E, bool RAG>
 static int launch_reg_epi(const Grid3 &g, const LineOpDev<R> &op, const SweepBatch<R> &b, const RhsFinalArgs<R> &rf,
                           int px, int py, int pz, cudaStream_t st) {
-    const int S = op.N / L;
+    const int S = (op.N + L - 1) / L;
     size_t smem = reg_smem_bytes(DIR, op.N, S, sizeof(R));
-    auto kern = sweep_reg_kernel<DIR, R, KIND, H, L, E>;
+    void (*kern)(Grid3, LineOpDev<R>, SweepBatch<R>, RhsFinalArgs<R>, int, int, int);
+    if constexpr (RAG) kern = sweep_rag_kernel<DIR, R, KIND, H, L, E>;
+    else kern = sweep_reg_kernel<DIR, R, KIND, H, L, E>;
     static KernelLaunchState ls;
     if (int rc = open_kernel(kern, ls, smem, 0, nullptr)) return rc;
     int tiles;
@@ -651,16 +828,16 @@ static int launch_reg_epi(const Grid3 &g, const LineOpDev<R> &op, const SweepBat
 // Epilogues instantiated per operator family: derivatives (H <= 3) store,
 // negate, accumulate or assemble k2; filters (H >= 4) store in the working
 // precision or in FP64. Other combinations go to the shared-memory kernels.
-template <int DIR, typename R, int KIND, int H, int L>
+template <int DIR, typename R, int KIND, int H, int L, bool RAG = false>
 static int launch_reg_one(const Grid3 &g, const LineOpDev<R> &op, const SweepBatch<R> &b, int epi,
                           const RhsFinalArgs<R> &rf, int px, int py, int pz, cudaStream_t st) {
-    if (epi == EPI_STORE) return launch_reg_epi<DIR, R, KIND, H, L, EPI_STORE>(g, op, b, rf, px, py, pz, st);
+    if (epi == EPI_STORE) return launch_reg_epi<DIR, R, KIND, H, L, EPI_STORE, RAG>(g, op, b, rf, px, py, pz, st);
     if constexpr (H <= 3) {
-        if (epi == EPI_STORE_NEG) return launch_reg_epi<DIR, R, KIND, H, L, EPI_STORE_NEG>(g, op, b, rf, px, py, pz, st);
-        if (epi == EPI_SUB) return launch_reg_epi<DIR, R, KIND, H, L, EPI_SUB>(g, op, b, rf, px, py, pz, st);
-        if (epi == EPI_RHS_FINAL) return launch_reg_epi<DIR, R, KIND, H, L, EPI_RHS_FINAL>(g, op, b, rf, px, py, pz, st);
+        if (epi == EPI_STORE_NEG) return launch_reg_epi<DIR, R, KIND, H, L, EPI_STORE_NEG, RAG>(g, op, b, rf, px, py, pz, st);
+        if (epi == EPI_SUB) return launch_reg_epi<DIR, R, KIND, H, L, EPI_SUB, RAG>(g, op, b, rf, px, py, pz, st);
+        if (epi == EPI_RHS_FINAL) return launch_reg_epi<DIR, R, KIND, H, L, EPI_RHS_FINAL, RAG>(g, op, b, rf, px, py, pz, st);
     } else {
-        if (epi == EPI_STORE_F64) return launch_reg_epi<DIR, R, KIND, H, L, EPI_STORE_F64>(g, op, b, rf, px, py, pz, st);
+        if (epi == EPI_STORE_F64) return launch_reg_epi<DIR, R, KIND, H, L, EPI_STORE_F64, RAG>(g, op, b, rf, px, py, pz, st);
     }
     return MC3D_ERR_CONFIG;
 }
@@ -697,6 +874,20 @@ int launch_sweep_reg(const Grid3 &g, const LineOpDev<R> &op, const SweepBatch<R>
     if constexpr (sizeof(R) == 4) {
         MC3D_RKINDS(64)
     }
+#undef MC3D_RCASE
+    return MC3D_ERR_CONFIG;
+}
+
+// The same for lines whose length is no multiple of the segment length.
+template <int DIR, typename R>
+int launch_sweep_rag(const Grid3 &g, const LineOpDev<R> &op, const SweepBatch<R> &b, int epi,
+                     const RhsFinalArgs<R> &rf, int px, int py, int pz, cudaStream_t st) {
+    // the FP32 solve of H <= 3, as in launch_sweep_reg
+    if (sizeof(R) == 4 && op.H <= 3 && (px || py || pz || !op.asym)) return MC3D_ERR_CONFIG;
+#define MC3D_RCASE(K, HH, LL)                                                  \
+    if (op.kind == K && op.H == HH && op.L == LL)                              \
+        return launch_reg_one<DIR, R, K, HH, LL, true>(g, op, b, epi, rf, px, py, pz, st);
+    MC3D_RKINDS(32)
 #undef MC3D_RKINDS
 #undef MC3D_RCASE
     return MC3D_ERR_CONFIG;

@@ -794,10 +794,10 @@ int launch_sweep(int dir, const Grid3 &g, const LineOpDev<R> &op, const SweepBat
     int py = filter_passthrough && bc_types[1] == MC3D_DIRICHLET_SOLVE;
     int pz = filter_passthrough && bc_types[2] == MC3D_DIRICHLET_SOLVE;
     if (op.L > 0 && g.n() < (1LL << 31) &&   // register-resident kernels index fields with 32-bit offsets
-        reg_smem_bytes(dir, op.N, op.N / op.L, sizeof(R)) <= 227 * 1024) {
-        int rc = dir == 0 ? launch_sweep_reg<0, R>(g, op, b, epi, rf, px, py, pz, st)
-                 : dir == 1 ? launch_sweep_reg<1, R>(g, op, b, epi, rf, px, py, pz, st)
-                            : launch_sweep_reg<2, R>(g, op, b, epi, rf, px, py, pz, st);
+        reg_smem_bytes(dir, op.N, (op.N + op.L - 1) / op.L, sizeof(R)) <= 227 * 1024) {
+        auto launch = op.rag ? (dir == 0 ? launch_sweep_rag<0, R> : dir == 1 ? launch_sweep_rag<1, R> : launch_sweep_rag<2, R>)
+                             : (dir == 0 ? launch_sweep_reg<0, R> : dir == 1 ? launch_sweep_reg<1, R> : launch_sweep_reg<2, R>);
+        const int rc = launch(g, op, b, epi, rf, px, py, pz, st);
         if (rc != MC3D_ERR_CONFIG) return rc;
     }
     size_t smem = ((size_t)(op.N + op.H + UB) * SP + 4 * W) * sizeof(R);

@@ -178,6 +178,66 @@ def test_register_kernel_pass_through_lines(prec, n):
             assert np.array_equal(out[tuple(face)], x.double().cpu().numpy()[tuple(face)]), (op, d)
 
 
+@pytest.mark.parametrize("prec", [m.FP64, m.FP32BULK])
+@pytest.mark.parametrize("bc", [m.PERIODIC_SOLVE, m.DIRICHLET_SOLVE])
+@pytest.mark.parametrize("n", [11, 16, 31, 32, 33, 34, 40, 63, 65, 97, 150, 257, 511])
+def test_ragged_lines_vs_oracle(n, bc, prec):
+    """Line lengths that are no multiple of the segment length (the ragged form
+    of the register-resident solve): one segment, a last segment of one row, of
+    two, of all but one, and 16 segments; every operator kind and direction, the
+    other dimensions not multiples of the 32-line tile, against the oracle."""
+    torch = _torch()
+    from oracle import mc3d_oracle as O
+    rng = np.random.default_rng(n + 7 * bc)
+    dt = torch.float64 if prec == m.FP64 else torch.float32
+    for d in range(3):
+        shape = [13, 19, 37]   # (13 x 19 x-lines: the last tile has 23)
+        shape[2 - d] = n
+        shape = tuple(shape)
+        f = rng.standard_normal(shape)
+        x = torch.tensor(f, dtype=dt, device="cuda")
+        bcs = [m.PERIODIC_SOLVE] * 3
+        bcs[d] = bc
+        for op in ("PADE6", "PENTA10", "COMPACT8", "COMPACT10", "TESTPADE"):
+            o = _make(op, d, bcs, shape, prec)
+            y = torch.empty_like(x)
+            if op.startswith("COMPACT"):
+                o.filterField(x, y)
+                ref = O.filt(f, d, op, G.OPS_ALPHA, tuple(bcs))
+            elif op == "TESTPADE":
+                o.filterField(x, y)
+                ref = O.test_filter(f, d, 1, tuple(bcs))
+            else:
+                o.calc1stDerivField(x, y)
+                ref = O.deriv(f, d, op, bc, 1.0 / n if bc == m.PERIODIC_SOLVE else 1.0 / (n - 1.0))
+            torch.cuda.synchronize()
+            err = H.rel_max(y.double().cpu().numpy(), ref)
+            assert err <= TOL[prec], (op, n, d, bc, err)
+
+
+@pytest.mark.parametrize("prec", [m.FP64, m.FP32BULK])
+def test_ragged_pass_through_lines(prec):
+    """Filter lines on the faces of walls pass through in the ragged solve."""
+    torch = _torch()
+    from oracle import mc3d_oracle as O
+    dt = torch.float64 if prec == m.FP64 else torch.float32
+    shape = (35, 49, 41)
+    f = np.random.default_rng(12).standard_normal(shape)
+    x = torch.tensor(f, dtype=dt, device="cuda")
+    for d in range(3):
+        bcs = [m.DIRICHLET_SOLVE] * 3
+        bcs[d] = m.PERIODIC_SOLVE
+        for op in ("COMPACT8", "COMPACT10"):
+            y = torch.empty_like(x)
+            _make(op, d, bcs, shape, prec).filterField(x, y)
+            ref = O.filt(f, d, op, G.OPS_ALPHA, tuple(bcs))
+            out = y.double().cpu().numpy()
+            assert H.rel_max(out, ref) <= TOL[prec], (op, d)
+            face = [slice(None)] * 3
+            face[2 - (d + 1) % 3] = 0
+            assert np.array_equal(out[tuple(face)], x.double().cpu().numpy()[tuple(face)]), (op, d)
+
+
 def test_tma_line_solves_complete_their_waits():
     """The TMA-staged FP32 line solves (256-point lines: persistent x and y/z
     kernels) finish without a bounded wait giving up, and agree with the
