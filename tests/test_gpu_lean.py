@@ -62,6 +62,24 @@ def test_lean_fp32bulk_holds_the_fp64_bound():
         assert H.rel_l2(q32[i], q64[i]) <= 1e-5, (i, H.rel_l2(q32[i], q64[i]))
 
 
+@pytest.mark.parametrize("prec,nx", [(m.FP64, 96), (m.FP64, 100), (m.FP64, 75), (m.FP32BULK, 75), (m.FP32BULK, 76),
+                                     (m.FP32BULK, 128), (m.FP32BULK, 320)])
+def test_lean_accumulates_along_x(prec, nx):
+    """The lean dataflow's accumulating x sweep in each of its kernels: bulk-copied
+    tiles of whole segments and of ragged lines (one copy a tile, one a line, and
+    blocks that end inside 16 bytes), TMA-staged FP32 lines of two and five
+    segments. Bounds as above."""
+    N = (nx, 25, 23)
+    ic = [np.ascontiguousarray(a[:, :, :nx]) for a in _ic((nx + nx % 2, 25, 23), 11)]   # (an even box)
+    q64, _ = _run("FULL", m.FP64, N, 4, ic)
+    q, _ = _run("LEAN", prec, N, 4, ic)
+    for i in range(5):
+        if prec == m.FP64:
+            assert H.rel_max(q[i], q64[i]) <= 1e-12, (nx, i, H.rel_max(q[i], q64[i]))
+        else:
+            assert H.rel_l2(q[i], q64[i]) <= 1e-5, (nx, i, H.rel_l2(q[i], q64[i]))
+
+
 def test_lean_learned_closure_runs_and_counts_out_of_range_stages():
     """LESMODEL = MLP with lean storage: no DSM fallback; stages that would have
     fallen back are counted. With a fallback fraction of 1 no stage counts and
