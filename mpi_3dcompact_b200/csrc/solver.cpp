@@ -27,6 +27,9 @@ struct mc3d_solver_s {
     mc3d_config cfg;
     int device = 0;
     cudaStream_t stream = nullptr;
+    // small blocks: the gradient sweeps' side streams and their events (gradients3)
+    cudaStream_t side[2] = {};
+    cudaEvent_t fork_ev = nullptr, join_ev[2] = {};
     mc3d::Grid3 g{};
     int prec = MC3D_FP64;
     double dxi[3] = {0, 0, 0};
@@ -112,6 +115,9 @@ static bool ragged_lines(int les_model, int precision) {
     return !(les_model == MC3D_DSM && precision != MC3D_FP64);
 }
 
+// Blocks up to this many points run their gradient sweeps side by side
+constexpr long long FORK_MAX_POINTS = 1LL << 20;
+
 // FP64 partial sums of GLOBAL averaging: up to 148 x 4 blocks for up to 8 fields
 constexpr size_t AVG_SCRATCH = 148 * 4 * 8;
 
@@ -184,7 +190,8 @@ const LineOpDev<double> &opdev<double>(const LineOpBuf &b) { return b.f64; }
 
 template <typename R>
 static int sweep_on(mc3d_solver s, const Grid3 &g, int dir, const LineOpBuf &op, int nf, const void *const *in,
-                    void *const *out, int epi, const void *const *aux, double *const *out64, bool filter, bool quirk);
+                    void *const *out, int epi, const void *const *aux, double *const *out64, bool filter, bool quirk,
+                    const cudaStream_t *on = nullptr);
 
 template <typename R>
 static int sweep(mc3d_solver s, int dir, const LineOpBuf &op, int nf, const void *const *in, void *const *out,
@@ -193,10 +200,12 @@ static int sweep(mc3d_solver s, int dir, const LineOpBuf &op, int nf, const void
 }
 
 // one batched line solve along dir over the block (or slab) g; `quirk` turns
-// on the momentum k2 carry-over of the k2-assembly epilogue
+// on the momentum k2 carry-over of the k2-assembly epilogue; *on, where given,
+// is the stream to launch on in place of the solver's (untimed launches only)
 template <typename R>
 static int sweep_on(mc3d_solver s, const Grid3 &g, int dir, const LineOpBuf &op, int nf, const void *const *in,
-                    void *const *out, int epi, const void *const *aux, double *const *out64, bool filter, bool quirk) {
+                    void *const *out, int epi, const void *const *aux, double *const *out64, bool filter, bool quirk,
+                    const cudaStream_t *on) {
     SweepBatch<R> b{};
     b.nf = nf;
     for (int f = 0; f < nf; f++) {
@@ -221,9 +230,33 @@ static int sweep_on(mc3d_solver s, const Grid3 &g, int dir, const LineOpBuf &op,
     if (epi == EPI_RHS_FINAL) bytes = (3.0 * nf + (quirk ? 3.0 : 0.0)) * sizeof(R) * (double)g.n();
     int rc = tic(s, KC_SWEEP, bytes);
     if (rc) return rc;
-    rc = launch_sweep<R>(dir, g, opdev<R>(op), b, epi, rf, s->cfg.bc_type, filter, s->stream);
+    rc = launch_sweep<R>(dir, g, opdev<R>(op), b, epi, rf, s->cfg.bc_type, filter, on ? *on : s->stream);
     if (rc) return rc;
     return toc(s);
+}
+
+// The first derivatives of nf fields along the three directions, out[d][f] from
+// in[f]. Blocks too small to fill the GPU run the directions side by side (they
+// read the same fields and write different ones): two streams fork from the
+// solver's stream and join it again before anything else is launched.
+template <typename R>
+static int gradients3(mc3d_solver s, int nf, void *const *in, void *const (*out)[4]) {
+    const bool fork = s->side[0] && !s->timing;
+    int rc;
+    if (fork) {
+        MC3D_CUDA_TRY(cudaEventRecord(s->fork_ev, s->stream));
+        for (int d = 0; d < 2; d++) MC3D_CUDA_TRY(cudaStreamWaitEvent(s->side[d], s->fork_ev, 0));
+    }
+    rc = MC3D_OK;
+    for (int d = 0; d < 3 && !rc; d++)
+        rc = sweep_on<R>(s, s->g, d, s->dop[d], nf, in, out[d], EPI_STORE, nullptr, nullptr, false,
+                         s->cfg.reference_quirks != 0, fork && d < 2 ? &s->side[d] : nullptr);
+    if (fork)   // (also after a failed launch: the solver's stream never runs ahead of the side streams)
+        for (int d = 0; d < 2; d++) {
+            MC3D_CUDA_TRY(cudaEventRecord(s->join_ev[d], s->side[d]));
+            MC3D_CUDA_TRY(cudaStreamWaitEvent(s->stream, s->join_ev[d], 0));
+        }
+    return rc;
 }
 
 // Three directional filter sweeps in the rotating order of
@@ -526,11 +559,10 @@ static int stage_rhs(mc3d_solver s, double *const *qP) {
     bool dsm = s->cfg.les_model == MC3D_DSM;
     // gradients of U, V, W, T in each direction: der[3*var + dir]; with DSM
     // the T gradient waits for the tau_kk correction of T
-    for (int d = 0; d < 3; d++) {
-        void *out[4] = {s->der[0 + d], s->der[3 + d], s->der[6 + d], s->der[9 + d]};
-        if ((rc = sweep<R>(s, d, s->dop[d], dsm ? 3 : 4, s->prim + 1, out, EPI_STORE, nullptr, nullptr, false)))
-            return rc;
-    }
+    void *grad[3][4];
+    for (int d = 0; d < 3; d++)
+        for (int v = 0; v < 4; v++) grad[d][v] = s->der[3 * v + d];
+    if ((rc = gradients3<R>(s, dsm ? 3 : 4, s->prim + 1, grad))) return rc;
     const R *pr[5];
     for (int v = 0; v < 5; v++) pr[v] = (const R *)s->prim[v];
     Metrics<R> m = metrics_of<R>(s);
@@ -580,10 +612,8 @@ static int stage_rhs(mc3d_solver s, double *const *qP) {
     }
     if (dsm) {
         if ((rc = dsm_mu_taukk<R>(s, qP, m))) return rc;
-        for (int d = 0; d < 3; d++) {
-            void *in[1] = {s->prim[4]}, *out[1] = {s->der[9 + d]};
-            if ((rc = sweep<R>(s, d, s->dop[d], 1, in, out, EPI_STORE, nullptr, nullptr, false))) return rc;
-        }
+        for (int d = 0; d < 3; d++) grad[d][0] = s->der[9 + d];
+        if ((rc = gradients3<R>(s, 1, s->prim + 4, grad))) return rc;
         if ((rc = dsm_ksgs<R>(s, qP, m))) return rc;
         fp.les = 3;
     }
@@ -977,6 +1007,17 @@ int mc3d_solver_create(const mc3d_config *cfg, int device, mc3d_solver *out) {
         delete s;
         return fail(MC3D_ERR_CUDA, std::string("cudaStreamCreate: ") + cudaGetErrorString(e));
     }
+    if ((long long)c.Nx * c.Ny * c.Nz <= FORK_MAX_POINTS) {
+        for (int d = 0; d < 2 && e == cudaSuccess; d++) {
+            e = cudaStreamCreateWithFlags(&s->side[d], cudaStreamNonBlocking);
+            if (e == cudaSuccess) e = cudaEventCreateWithFlags(&s->join_ev[d], cudaEventDisableTiming);
+        }
+        if (e == cudaSuccess) e = cudaEventCreateWithFlags(&s->fork_ev, cudaEventDisableTiming);
+        if (e != cudaSuccess) {
+            mc3d_solver_destroy(s);
+            return fail(MC3D_ERR_CUDA, std::string("side streams: ") + cudaGetErrorString(e));
+        }
+    }
     int N[3] = {c.Nx, c.Ny, c.Nz};
     int rc = MC3D_OK;
     try {
@@ -1104,6 +1145,11 @@ int mc3d_solver_destroy(mc3d_solver s) {
     if (!s) return MC3D_OK;
     cudaSetDevice(s->device);
     if (s->stream) cudaStreamSynchronize(s->stream);
+    for (int d = 0; d < 2; d++) {
+        if (s->side[d]) cudaStreamDestroy(s->side[d]);
+        if (s->join_ev[d]) cudaEventDestroy(s->join_ev[d]);
+    }
+    if (s->fork_ev) cudaEventDestroy(s->fork_ev);
     for (cudaEvent_t e : s->events) cudaEventDestroy(e);
     for (void *p : s->allocs) cudaFree(p);
     if (s->mlp_flag_host) cudaFreeHost(s->mlp_flag_host);
