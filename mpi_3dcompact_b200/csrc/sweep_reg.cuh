@@ -189,59 +189,6 @@ __device__ __forceinline__ void reg_copy_out(const SweepBatch<R> &b, const RhsFi
     }
 }
 
-// x lines of any length: the tile's nl lines go round the S warps, each line's
-// values round the lanes (whole lines, so that rows of any length stay
-// contiguous across the warp); the read operands of four groups of 32 values
-// are loaded before the groups' stores.
-template <typename R, int E>
-__device__ __forceinline__ void rag_copy_out(const SweepBatch<R> &b, const RhsFinalArgs<R> &rf, int f, int tile0,
-                                             int N, int nl, int seg, int S, int lane, const R *tile) {
-    constexpr int P = W + 1;
-    constexpr int G = 4;
-    constexpr bool RD_OLD = E == EPI_SUB || E == EPI_RHS_FINAL;
-    constexpr bool RD_AUX = E == EPI_RHS_FINAL;
-    const R dt = (E == EPI_RHS_FINAL) ? (R)(*rf.dt) : R(0);
-    const bool mom = (E == EPI_RHS_FINAL) && rf.quirk && b.eq[f] >= 1 && b.eq[f] <= 3;
-    const bool rd_old = E == EPI_SUB || mom;
-    R *o = b.out[f];
-    double *o64 = b.out64[f];
-    const R *ax = b.aux[f];
-    const R *jp = rf.J;
-    for (int l = seg; l < nl; l += S) {
-        const int line0 = (tile0 + l) * N;
-        for (int i0 = 0; i0 < N; i0 += 32 * G) {
-            R old[G], aux[G], jj[G];
-#pragma unroll
-            for (int q = 0; q < G; q++) {
-                const int i = i0 + 32 * q + lane;
-                if (i < N) {
-                    if (RD_OLD) old[q] = rd_old ? o[line0 + i] : R(0);
-                    if (RD_AUX) {
-                        aux[q] = ax[line0 + i];
-                        jj[q] = jp ? jp[line0 + i] : rf.Jc;
-                    }
-                }
-            }
-#pragma unroll
-            for (int q = 0; q < G; q++) {
-                const int i = i0 + 32 * q + lane;
-                if (i >= N) break;
-                const int off = line0 + i;
-                const R v = tile[i * P + l];
-                if (E == EPI_STORE) o[off] = v;
-                if (E == EPI_STORE_NEG) o[off] = -v;
-                if (E == EPI_SUB) o[off] = old[q] - v;
-                if (E == EPI_STORE_F64) o64[off] = (double)v;
-                if (E == EPI_RHS_FINAL) {
-                    R tt = aux[q] - v;
-                    R dtJ = dt * jj[q];
-                    o[off] = mom ? (old[q] + tt) * dtJ : tt * dtJ;
-                }
-            }
-        }
-    }
-}
-
 // E: the caller's operation (EpiMode), compiled into the kernel so that each
 // instantiation carries one epilogue only.
 // The solve of one tile once each lane holds rows a-H .. a+L+H-1 of its line
@@ -716,92 +663,199 @@ __global__ void __launch_bounds__(512) sweep_reg_kernel(Grid3 g, LineOpDev<R> op
     }
 }
 
-// Lines whose length is no multiple of the segment length (the RAG form of
-// reg_solve): S = ceil(N / L) warps, the last with the rows that are left.
-// Bound by the latency of the recurrences, like the other line solves; the
-// whole-line kernel that served these lengths before (one warp a tile, every
-// recurrence over all N rows, each row through shared memory) kept 8 warps an
-// SM busy where this keeps 16.
+// rows a-H .. a+L+H-1 of a ragged line into v by row(n), n in [0, N): periodic
+// wrap, or zero outside the line and for the last segment's rows past the wrap.
+template <typename R, int KIND, int H, int L, typename Row>
+__device__ __forceinline__ void rag_load_rows(int a, int N, const Row &row, R (&v)[L + 2 * H]) {
+    constexpr bool PER = (KIND % 2) == 0;
+    constexpr int NV = L + 2 * H;
+    if (a >= H && a + L + H <= N) {
+#pragma unroll
+        for (int k = 0; k < NV; k++) v[k] = row(a - H + k);
+        return;
+    }
+#pragma unroll
+    for (int k = 0; k < NV; k++) {
+        int n = a - H + k;
+        bool in = true;
+        if (n < 0) {
+            n += N;
+            in = PER;
+        } else if (n >= N) {
+            n -= N;
+            in = PER && n < H;
+        }
+        v[k] = in ? row(n) : R(0);
+    }
+}
+
+// y and z lines whose length is no multiple of L (the RAG form of reg_solve):
+// S = ceil(N / L) warps, the last with the rows that are left. Bound by the
+// latency of the recurrences; the whole-line kernel that served such lengths
+// before kept one warp a tile busy with N-row recurrences through shared memory
+// (FP64 y derivatives of four 84 x 187 x 146 fields: 91 us there, 55 us here).
 template <int DIR, typename R, int KIND, int H, int L, int E>
 __global__ void __launch_bounds__(512) sweep_rag_kernel(Grid3 g, LineOpDev<R> op, SweepBatch<R> b,
                                                         RhsFinalArgs<R> rf, int pass_y, int pass_z, int pass_x) {
-    constexpr bool PER = (KIND % 2) == 0;
-    constexpr int NV = L + 2 * H;
-    constexpr int P = W + 1;
+    static_assert(DIR == 1 || DIR == 2, "x lines: sweep_rag_x_kernel");
     extern __shared__ __align__(16) unsigned char smem_raw[];
     R *sh = reinterpret_cast<R *>(smem_raw);
     const int S = blockDim.x >> 5;
     const int lane = threadIdx.x & 31, seg = threadIdx.x >> 5;
     const int N = op.N, a = seg * L;
-    const int Lw = N - a < L ? N - a : L;
     const int f = blockIdx.y;
-    R *tile = sh + reg_chain_elems(S);   // x lines: [N][W+1], after the chain states
 
     const TileGeom t = tile_geom<DIR>(g, blockIdx.x, lane);
     bool pass = false;
-    if (DIR == 0) pass = (pass_y && (t.j == 0 || t.j == g.Ny - 1)) || (pass_z && (t.k == 0 || t.k == g.Nz - 1));
     if (DIR == 1) pass = (pass_x && (t.i == 0 || t.i == g.Nx - 1)) || (pass_z && (t.k == 0 || t.k == g.Nz - 1));
     if (DIR == 2) pass = (pass_y && (t.j == 0 || t.j == g.Ny - 1)) || (pass_x && (t.i == 0 || t.i == g.Nx - 1));
     const bool work = t.active && !pass;
 
-    // ---- load rows a-H .. a+L+H-1 of this lane's line (periodic wrap / zero) ----
-    int nl = W;
-    const R *src;
-    if (DIR == 0) {
-        const long long rem = (long long)g.Ny * g.Nz - (long long)blockIdx.x * W;
-        nl = rem < W ? (int)rem : W;
-        src = b.in[f] + (size_t)blockIdx.x * W * N;
-        // the lines go round the warps, each line's values round the lanes
-        for (int l = seg; l < nl; l += S)
-            for (int i = lane; i < N; i += 32) cp_async_elem(&tile[i * P + l], src + l * N + i);
-        cp_async_wait_all();
-        __syncthreads();
-    } else {
-        src = b.in[f] + (int)t.base;
-    }
+    const R *src = b.in[f] + (int)t.base;
     const int stride = (int)t.stride;
-    auto row = [&](int n) -> R {
-        if (DIR == 0) return tile[n * P + lane];
-        return t.active ? src[n * stride] : R(0);
-    };
-    R v[NV];
-    if (a >= H && a + L + H <= N) {
-#pragma unroll
-        for (int k = 0; k < NV; k++) v[k] = row(a - H + k);
-    } else {
-#pragma unroll
-        for (int k = 0; k < NV; k++) {
-            int n = a - H + k;
-            bool in = true;
-            if (n < 0) {
-                n += N;
-                in = PER;
-            } else if (n >= N) {
-                n -= N;
-                in = PER && n < H;
-            }
-            v[k] = in ? row(n) : R(0);
-        }
-    }
+    auto row = [&](int n) -> R { return t.active ? src[n * stride] : R(0); };
+    R v[L + 2 * H];
+    rag_load_rows<R, KIND, H, L>(a, N, row, v);
 
     R y[L];
     reg_solve<R, KIND, H, L, false, NoFwdHook, true>(op, v, y, work, lane, seg, S, a, sh, NoFwdHook(),
-                                                     [&](int k) { return row(N - MC3D_BWMAX + k); });
+                                                    [&](int k) { return row(N - MC3D_BWMAX + k); });
 
-    // ---- epilogue ----
-    if (DIR == 0) {
-        // (every lane's line values were read before the solve's barriers)
-        if (t.active) {
-#pragma unroll
-            for (int r = 0; r < L; r++)
-                if (r < Lw) tile[(a + r) * P + lane] = y[r];
-        }
-        __syncthreads();
-        rag_copy_out<R, E>(b, rf, f, (int)blockIdx.x * W, N, nl, seg, S, lane, tile);
-    } else if (t.active) {
+    if (t.active) {
         const int off0 = (int)t.base + a * stride;
-        if (Lw == L) reg_store_rows<R, E, L>(b, rf, f, off0, stride, y);
-        else reg_store_rows<R, E, L, true, true>(b, rf, f, off0, stride, y, Lw);
+        if (a + L <= N) reg_store_rows<R, E, L>(b, rf, f, off0, stride, y);
+        else reg_store_rows<R, E, L, true, true>(b, rf, f, off0, stride, y, N - a);
+    }
+}
+
+// Pitch of a line in the x tile: the field's own where lines are no multiple of
+// 16 bytes or an odd number of 16-byte units, else one unit more, so that the
+// lanes' lines fall into different banks.
+__host__ __device__ inline int x_pitch(int N, int esize) {
+    const int bytes = N * esize;
+    return bytes % 16 == 0 && (bytes / 16) % 2 == 0 ? N + 16 / esize : N;
+}
+inline size_t x_smem_bytes(int N, int S, size_t esize) {
+    return (size_t)W * x_pitch(N, (int)esize) * esize + (size_t)reg_chain_elems(S) * esize;
+}
+
+// CTAs whose wait for a bulk copy gave up (one counter a translation unit)
+static __device__ int g_bulk_wait_timeouts;
+
+// Ragged x lines: the tile's 32 lines are one contiguous block of the field, brought
+// into shared memory by bulk copies (one for the block, or one a line where the
+// tile's pitch differs), read and overwritten by each lane along its own line,
+// and stored by bulk copies: no instruction per element but the lane's own
+// shared loads and stores. The accumulating sweep's operand takes the tile
+// while the lanes solve. Against a transposed tile filled by one cp.async per
+// element: three-direction gradients of four FP64 fields of 150 x 97 x 75 107 us
+// / 97 us, channel step of 100 x 97 x 60 907 us / 871 us. Lines of whole segments
+// keep the transposed tile: their even pitches make four lanes share a bank
+// (64^3 FP64 step 410 us there, 442 us here).
+template <typename R, int KIND, int H, int L, int E>
+__global__ void __launch_bounds__(512) sweep_rag_x_kernel(Grid3 g, LineOpDev<R> op, SweepBatch<R> b, int pass_y,
+                                                      int pass_z) {
+    static_assert(E != EPI_RHS_FINAL, "the k2 assembly runs along z");
+    extern __shared__ __align__(128) unsigned char smem_raw[];
+    __shared__ __align__(8) unsigned long long bar;
+    R *tile = reinterpret_cast<R *>(smem_raw);
+    const int N = op.N, P = x_pitch(N, (int)sizeof(R));
+    R *sh = tile + W * P;
+    const int S = blockDim.x >> 5;
+    const int lane = threadIdx.x & 31, seg = threadIdx.x >> 5, a = seg * L;
+    const int f = blockIdx.y;
+    const size_t first = (size_t)blockIdx.x * W * N;
+    const long long rem = (long long)g.Ny * g.Nz - (long long)blockIdx.x * W;
+    const int nl = rem < W ? (int)rem : W;
+    const unsigned bar_a = (unsigned)__cvta_generic_to_shared(&bar);
+    const unsigned tile_a = (unsigned)__cvta_generic_to_shared(tile);
+    const unsigned total = (unsigned)(nl * N) * (unsigned)sizeof(R), line = (unsigned)N * (unsigned)sizeof(R);
+    // (a block of fewer than 32 lines may end inside a 16-byte unit: those
+    // values go one by one)
+    const unsigned whole = P == N ? total & ~15u : total;
+    const int tail0 = (int)(whole / sizeof(R)), tail1 = P == N ? nl * N : tail0;
+    auto load = [&](const R *src) {   // warp 0
+        if (lane == 0)
+            asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar_a), "r"(whole) : "memory");
+        __syncwarp();
+        if (P == N ? lane == 0 && whole > 0 : lane < nl)
+            asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                             tile_a + (unsigned)(lane * P) * (unsigned)sizeof(R)),
+                         "l"(src + (size_t)lane * N), "r"(P == N ? whole : line), "r"(bar_a)
+                         : "memory");
+        if (tail0 + lane < tail1) tile[tail0 + lane] = src[tail0 + lane];
+    };
+    // bounded wait for the phase of the given parity; the CTA decides together
+    auto wait = [&](unsigned parity) -> bool {
+        unsigned done = 0;
+        for (int it = 0; it < (1 << 22) && !done; it++)
+            asm volatile(
+                "{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}"
+                : "=r"(done)
+                : "r"(bar_a), "r"(parity)
+                : "memory");
+        if (__syncthreads_and(done != 0)) return true;
+        if (threadIdx.x == 0) atomicAdd(&g_bulk_wait_timeouts, 1);
+        return false;
+    };
+    if (threadIdx.x == 0) {
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar_a) : "memory");
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (seg == 0) {
+        __syncwarp();
+        load(b.in[f] + first);
+    }
+    __syncthreads();
+    if (!wait(0)) return;
+
+    const TileGeom t = tile_geom<0>(g, blockIdx.x, lane);
+    const bool pass = (pass_y && (t.j == 0 || t.j == g.Ny - 1)) || (pass_z && (t.k == 0 || t.k == g.Nz - 1));
+    R *mine = tile + lane * P;
+    auto row = [&](int n) -> R { return mine[n]; };
+    R v[L + 2 * H];
+    rag_load_rows<R, KIND, H, L>(a, N, row, v);
+    R tailv[MC3D_BWMAX];
+    if ((KIND % 2) == 1 && a + L > N - H) {
+#pragma unroll
+        for (int k = 0; k < MC3D_BWMAX; k++) tailv[k] = row(N - MC3D_BWMAX + k);
+    }
+    auto refill = [&](int ph) {
+        if (E != EPI_SUB) return;
+        if (ph == 0) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // this thread's reads of the tile
+        else if (seg == 0) load(b.out[f] + first);
+    };
+    R y[L];
+    reg_solve<R, KIND, H, L, false, decltype(refill), true>(op, v, y, t.active && !pass, lane, seg, S, a, sh, refill,
+                                                           [&](int k) { return tailv[k]; });
+    if (E == EPI_SUB && !wait(1)) return;
+    if (t.active) {
+#pragma unroll
+        for (int r = 0; r < L; r++) {
+            if (a + r >= N) break;
+            mine[a + r] = E == EPI_SUB ? mine[a + r] - y[r] : E == EPI_STORE_NEG ? -y[r] : y[r];
+        }
+    }
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    __syncthreads();
+    if constexpr (E == EPI_STORE_F64 && sizeof(R) == 4) {
+        // widened on the way out: the lines go round the warps, their values round the lanes
+        for (int l = seg; l < nl; l += S) {
+            double *o = b.out64[f] + first + (size_t)l * N;
+#pragma unroll 4
+            for (int n = lane; n < N; n += 32) o[n] = (double)tile[l * P + n];
+        }
+    } else if (seg == 0) {
+        R *dst;
+        if constexpr (E == EPI_STORE_F64) dst = b.out64[f] + first;
+        else dst = b.out[f] + first;
+        if (P == N ? lane == 0 && whole > 0 : lane < nl)
+            asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(dst + (size_t)lane * N),
+                         "r"(tile_a + (unsigned)(lane * P) * (unsigned)sizeof(R)), "r"(P == N ? whole : line)
+                         : "memory");
+        if (tail0 + lane < tail1) dst[tail0 + lane] = tile[tail0 + lane];
+        asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+        asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
     }
 }
 
@@ -809,18 +863,21 @@ template <int DIR, typename R, int KIND, int H, int L, int E, bool RAG>
 static int launch_reg_epi(const Grid3 &g, const LineOpDev<R> &op, const SweepBatch<R> &b, const RhsFinalArgs<R> &rf,
                           int px, int py, int pz, cudaStream_t st) {
     const int S = (op.N + L - 1) / L;
-    size_t smem = reg_smem_bytes(DIR, op.N, S, sizeof(R));
-    void (*kern)(Grid3, LineOpDev<R>, SweepBatch<R>, RhsFinalArgs<R>, int, int, int);
-    if constexpr (RAG) kern = sweep_rag_kernel<DIR, R, KIND, H, L, E>;
-    else kern = sweep_reg_kernel<DIR, R, KIND, H, L, E>;
     static KernelLaunchState ls;
-    if (int rc = open_kernel(kern, ls, smem, 0, nullptr)) return rc;
-    int tiles;
-    if (DIR == 0) tiles = (int)(((long long)g.Ny * g.Nz + W - 1) / W);
-    else if (DIR == 1) tiles = ((g.Nx + W - 1) / W) * g.Nz;
-    else tiles = (int)(((long long)g.Nx * g.Ny + W - 1) / W);
-    dim3 grid(tiles, b.nf);
-    kern<<<grid, 32 * S, smem, st>>>(g, op, b, rf, py, pz, px);
+    const dim3 grid(tile_count<DIR>(g), b.nf);
+    if constexpr (RAG && DIR == 0) {
+        const size_t smem = x_smem_bytes(op.N, S, sizeof(R));
+        auto kern = sweep_rag_x_kernel<R, KIND, H, L, E>;
+        if (int rc = open_kernel(kern, ls, smem, 0, nullptr)) return rc;
+        kern<<<grid, 32 * S, smem, st>>>(g, op, b, py, pz);
+    } else {
+        const size_t smem = reg_smem_bytes(DIR, op.N, S, sizeof(R));
+        void (*kern)(Grid3, LineOpDev<R>, SweepBatch<R>, RhsFinalArgs<R>, int, int, int);
+        if constexpr (RAG) kern = sweep_rag_kernel<DIR, R, KIND, H, L, E>;
+        else kern = sweep_reg_kernel<DIR, R, KIND, H, L, E>;
+        if (int rc = open_kernel(kern, ls, smem, 0, nullptr)) return rc;
+        kern<<<grid, 32 * S, smem, st>>>(g, op, b, rf, py, pz, px);
+    }
     MC3D_CUDA_TRY(cudaGetLastError());
     return MC3D_OK;
 }
@@ -831,11 +888,20 @@ static int launch_reg_epi(const Grid3 &g, const LineOpDev<R> &op, const SweepBat
 template <int DIR, typename R, int KIND, int H, int L, bool RAG = false>
 static int launch_reg_one(const Grid3 &g, const LineOpDev<R> &op, const SweepBatch<R> &b, int epi,
                           const RhsFinalArgs<R> &rf, int px, int py, int pz, cudaStream_t st) {
+    if constexpr (RAG && DIR == 0) {   // bulk copies start and end on 16-byte boundaries
+        const bool f64 = epi == EPI_STORE_F64;
+        for (int f = 0; f < b.nf; f++)
+            if ((((uintptr_t)b.in[f] | (f64 ? (uintptr_t)b.out64[f] : (uintptr_t)b.out[f])) & 15) != 0)
+                return MC3D_ERR_CONFIG;
+    }
     if (epi == EPI_STORE) return launch_reg_epi<DIR, R, KIND, H, L, EPI_STORE, RAG>(g, op, b, rf, px, py, pz, st);
     if constexpr (H <= 3) {
         if (epi == EPI_STORE_NEG) return launch_reg_epi<DIR, R, KIND, H, L, EPI_STORE_NEG, RAG>(g, op, b, rf, px, py, pz, st);
         if (epi == EPI_SUB) return launch_reg_epi<DIR, R, KIND, H, L, EPI_SUB, RAG>(g, op, b, rf, px, py, pz, st);
-        if (epi == EPI_RHS_FINAL) return launch_reg_epi<DIR, R, KIND, H, L, EPI_RHS_FINAL, RAG>(g, op, b, rf, px, py, pz, st);
+        if constexpr (!(RAG && DIR == 0)) {   // (the k2 assembly runs along z)
+            if (epi == EPI_RHS_FINAL)
+                return launch_reg_epi<DIR, R, KIND, H, L, EPI_RHS_FINAL, RAG>(g, op, b, rf, px, py, pz, st);
+        }
     } else {
         if (epi == EPI_STORE_F64) return launch_reg_epi<DIR, R, KIND, H, L, EPI_STORE_F64, RAG>(g, op, b, rf, px, py, pz, st);
     }

@@ -241,9 +241,10 @@ int tma_wait_timeouts(int *count) {
 extern "C" int mc3d_tma_wait_timeouts(int device, int *count) {
     if (!count) return mc3d::fail(MC3D_ERR_ARG, "null argument");
     MC3D_CUDA_TRY(cudaSetDevice(device));
-    int a = 0, b = 0;
-    if (int rc = mc3d::tma_wait_timeouts(&a)) return rc;
-    if (int rc = mc3d::mlp_wait_timeouts(&b)) return rc;
-    *count = a + b;
+    int n[3] = {0, 0, 0};
+    if (int rc = mc3d::tma_wait_timeouts(&n[0])) return rc;
+    if (int rc = mc3d::mlp_wait_timeouts(&n[1])) return rc;
+    if (int rc = mc3d::x_wait_timeouts_rag(&n[2])) return rc;
+    *count = n[0] + n[1] + n[2];
     return MC3D_OK;
 }
