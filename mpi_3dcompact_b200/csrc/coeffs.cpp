@@ -622,6 +622,7 @@ void fill_dev(const LineOpHost &h, const char *base, const Layout &lo, LineOpDev
     d.sbb = h.S > 1 ? sg + 3 * n : nullptr;
     d.L = h.L;
     d.rag = h.rag;
+    d.keep = h.keep;
     d.pf = h.L ? p + lo.pf : nullptr;
     d.pb = h.L ? p + lo.pb : nullptr;
     d.pz = h.L && h.kind == K_PEN_PER ? p + lo.pz : nullptr;
@@ -747,6 +748,7 @@ int upload_line_op(const LineOpHost &hin, int precision, LineOpBuf &out, bool ra
     if (h.bw > MC3D_BWMAX) return fail(MC3D_ERR_CONFIG, "boundary row wider than the kernels support");
     analyse(h, precision);
     segment(h, precision, ragged);
+    h.keep = !ragged;
     if (h.S > 1) {
         // responses below 2^-64 (FP64) / 2^-32 (FP32) of their unit start are dropped
         const double thr = std::ldexp(1.0, precision == MC3D_FP64 ? -64 : -32);

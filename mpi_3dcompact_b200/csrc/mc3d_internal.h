@@ -104,6 +104,7 @@ struct LineOpHost {
     int seg_kf = 0, seg_kb = 0;
     int L = 0;   // segment length of the register-resident kernel (0: not used)
     bool rag = false;   // N is no multiple of L: the last segment has fewer rows
+    bool keep = false;  // uploaded without `ragged`: keep the order (and contraction) of the sums
 };
 
 // Segment length of the register-resident line solve for a line of N points
@@ -150,6 +151,7 @@ struct LineOpDev {
     //   phi[0..BWMAX-1], tail right-aligned on phi[N-BWMAX..N-1])
     int L;
     int rag;   // N is no multiple of L: the last of ceil(N / L) segments has fewer rows
+    int keep;  // long FP32 x lines stay with the register kernel (upload_line_op without `ragged`)
     const R *pf, *pb, *pz, *sf2, *sb2, *hp, *tp;
     // FP32 derivative form of the register-resident solve (H <= 3): asym is 1
     // when the interior stencil is antisymmetric with a zero centre, sta[k-1]

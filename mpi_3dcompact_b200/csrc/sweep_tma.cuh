@@ -325,6 +325,144 @@ __global__ void __launch_bounds__(512) sweep_tma_yz_persist_kernel(Grid3 g, Line
     }
 }
 
+// rows a-H .. a+L+H-1 of line `lane` from a swizzled x tile (periodic wrap / zero)
+template <int KIND, int H, int L>
+__device__ __forceinline__ void tma_x_rows(const unsigned char *tile, int lane, int a, int N, float (&v)[L + 2 * H]) {
+    constexpr bool PER = (KIND % 2) == 0;
+    constexpr int NV = L + 2 * H;
+    constexpr int HC = (H + 3) / 4;
+#pragma unroll
+    for (int q = 0; q < L / 4; q++) {
+        const float4 x4 = lds4(tile, swz_off(lane, a + 4 * q));
+        v[H + 4 * q + 0] = x4.x;
+        v[H + 4 * q + 1] = x4.y;
+        v[H + 4 * q + 2] = x4.z;
+        v[H + 4 * q + 3] = x4.w;
+    }
+#pragma unroll
+    for (int hc = 0; hc < HC; hc++) {
+        int n = a - 4 * (hc + 1);
+        bool in = true;
+        if (n < 0) {
+            n += N;
+            in = PER;
+        }
+        const float4 x4 = in ? lds4(tile, swz_off(lane, n)) : make_float4(0.f, 0.f, 0.f, 0.f);
+        const float e[4] = {x4.x, x4.y, x4.z, x4.w};
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            const int k = H - 4 * (hc + 1) + j;
+            if (k >= 0) v[k] = e[j];
+        }
+        int m = a + L + 4 * hc;
+        bool in2 = true;
+        if (m >= N) {
+            m -= N;
+            in2 = PER;
+        }
+        const float4 x5 = in2 ? lds4(tile, swz_off(lane, m)) : make_float4(0.f, 0.f, 0.f, 0.f);
+        const float e2[4] = {x5.x, x5.y, x5.z, x5.w};
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            const int k = H + L + 4 * hc + j;
+            if (k < NV) v[k] = e2[j];
+        }
+    }
+}
+
+// x lines too long for the persistent kernel's two tiles, and the accumulating
+// sweep: one CTA per tile and one tile, which takes the previous output (the
+// accumulate's operand) while the lanes solve and then the results, which leave
+// by TMA store. Against the register kernel this replaces one asynchronous copy,
+// one transposed shared store and load and one global store per element with
+// bulk copies and 16-byte shared accesses (COMPACT10 of five 512 x 256 x 64
+// fields in three directions: 319 us there, 300 us here).
+template <int KIND, int H, int L, int E>
+__global__ void __launch_bounds__(512) sweep_tma_x_kernel(Grid3 g, LineOpDev<float> op,
+                                                          const __grid_constant__ TmaMaps maps, int pass_y,
+                                                          int pass_z) {
+    using R = float;
+    extern __shared__ __align__(1024) unsigned char smem_raw[];
+    __shared__ __align__(8) unsigned long long bar;
+    const unsigned base = smem_u32(smem_raw);
+    unsigned char *tile = smem_raw + ((1024u - (base & 1023u)) & 1023u);
+    const int N = op.N, nbox = N / TMA_BOX;
+    R *sh = reinterpret_cast<R *>(tile + nbox * 4096);
+    const int S = blockDim.x >> 5;
+    const int lane = threadIdx.x & 31, seg = threadIdx.x >> 5, a = seg * L;
+    const int tl = blockIdx.x, f = blockIdx.y;
+    const unsigned bar_a = smem_u32(&bar);
+    auto load = [&](const CUtensorMap *m) {
+        const unsigned long long tm = reinterpret_cast<unsigned long long>(m);
+        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar_a), "r"(nbox * 4096)
+                     : "memory");
+        for (int bx = 0; bx < nbox; bx++)
+            asm volatile(
+                "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], "
+                "[%4];" ::"r"(smem_u32(tile + bx * 4096)),
+                "l"(tm), "r"(bx * TMA_BOX), "r"(tl * W), "r"(bar_a)
+                : "memory");
+    };
+    // bounded wait for the phase of the given parity; the CTA decides together
+    auto wait = [&](unsigned parity) -> bool {
+        unsigned done = 0;
+        for (int it = 0; it < (1 << 22) && !done; it++)
+            asm volatile(
+                "{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}"
+                : "=r"(done)
+                : "r"(bar_a), "r"(parity)
+                : "memory");
+        if (__syncthreads_and(done != 0)) return true;
+        if (threadIdx.x == 0) atomicAdd(&g_tma_wait_timeouts, 1);
+        return false;
+    };
+    if (threadIdx.x == 0) {
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar_a) : "memory");
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        load(&maps.in[f]);
+    }
+    __syncthreads();
+    if (!wait(0)) return;
+
+    const TileGeom t = tile_geom<0>(g, tl, lane);
+    const bool pass = (pass_y && (t.j == 0 || t.j == g.Ny - 1)) || (pass_z && (t.k == 0 || t.k == g.Nz - 1));
+    R v[L + 2 * H];
+    tma_x_rows<KIND, H, L>(tile, lane, a, N, v);
+    // the tile is read: at the barrier that ends pass 1 it takes the operand
+    // (the results are written after the solve's second barrier)
+    auto refill = [&](int ph) {
+        if (E != EPI_SUB) return;
+        if (ph == 0) tile_reads_done();
+        else if (threadIdx.x == 0) load(&maps.out[f]);
+    };
+    R y[L];
+    reg_solve<R, KIND, H, L, E == EPI_STORE_NEG>(op, v, y, t.active && !pass, lane, seg, S, a, sh, refill);
+    if (E == EPI_SUB && !wait(1)) return;
+    if (t.active) {
+#pragma unroll
+        for (int q = 0; q < L / 4; q++) {
+            float4 *at = reinterpret_cast<float4 *>(tile + swz_off(lane, a + 4 * q));
+            float4 o4 = make_float4(y[4 * q + 0], y[4 * q + 1], y[4 * q + 2], y[4 * q + 3]);
+            if (E == EPI_SUB) {
+                const float4 old = *at;
+                o4 = make_float4(old.x - o4.x, old.y - o4.y, old.z - o4.z, old.w - o4.w);
+            }
+            *at = o4;
+        }
+    }
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        const unsigned long long tm = reinterpret_cast<unsigned long long>(&maps.out[f]);
+        for (int bx = 0; bx < nbox; bx++)
+            asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.tile.bulk_group [%0, {%1, %2}], [%3];" ::"l"(tm),
+                         "r"(bx * TMA_BOX), "r"(tl * W), "r"(smem_u32(tile + bx * 4096))
+                         : "memory");
+        asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+        asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+    }
+}
+
 // Persistent form of the x kernel: each CTA walks the (field, tile) items
 // gridDim.x apart with two tiles, one receiving the next item's TMA load
 // while the lanes solve the current one, the other holding the solution rows
@@ -335,9 +473,7 @@ __global__ void __launch_bounds__(512) sweep_tma_x_persist_kernel(Grid3 g, LineO
                                                                   const __grid_constant__ TmaMaps maps, int nf,
                                                                   int pass_y, int pass_z) {
     using R = float;
-    constexpr bool PER = (KIND % 2) == 0;
     constexpr int NV = L + 2 * H;
-    constexpr int HC = (H + 3) / 4;
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     __shared__ __align__(8) unsigned long long bar;
     const unsigned base = smem_u32(smem_raw);
@@ -390,43 +526,7 @@ __global__ void __launch_bounds__(512) sweep_tma_x_persist_kernel(Grid3 g, LineO
         const bool pass = (pass_y && (t.j == 0 || t.j == g.Ny - 1)) || (pass_z && (t.k == 0 || t.k == g.Nz - 1));
         const bool work = t.active && !pass;
         R v[NV];
-#pragma unroll
-        for (int q = 0; q < L / 4; q++) {
-            const float4 x4 = lds4(tin, swz_off(lane, a + 4 * q));
-            v[H + 4 * q + 0] = x4.x;
-            v[H + 4 * q + 1] = x4.y;
-            v[H + 4 * q + 2] = x4.z;
-            v[H + 4 * q + 3] = x4.w;
-        }
-#pragma unroll
-        for (int hc = 0; hc < HC; hc++) {
-            int n = a - 4 * (hc + 1);
-            bool in = true;
-            if (n < 0) {
-                n += N;
-                in = PER;
-            }
-            const float4 x4 = in ? lds4(tin, swz_off(lane, n)) : make_float4(0.f, 0.f, 0.f, 0.f);
-            const R e[4] = {x4.x, x4.y, x4.z, x4.w};
-#pragma unroll
-            for (int j = 0; j < 4; j++) {
-                const int k = H - 4 * (hc + 1) + j;
-                if (k >= 0) v[k] = e[j];
-            }
-            int m = a + L + 4 * hc;
-            bool in2 = true;
-            if (m >= N) {
-                m -= N;
-                in2 = PER;
-            }
-            const float4 x5 = in2 ? lds4(tin, swz_off(lane, m)) : make_float4(0.f, 0.f, 0.f, 0.f);
-            const R e2[4] = {x5.x, x5.y, x5.z, x5.w};
-#pragma unroll
-            for (int j = 0; j < 4; j++) {
-                const int k = H + L + 4 * hc + j;
-                if (k < NV) v[k] = e2[j];
-            }
-        }
+        tma_x_rows<KIND, H, L>(tin, lane, a, N, v);
         // the input tile takes the next item at the barrier that ends pass 1;
         // the output tile is written after the solve's second barrier, which
         // the issuing thread reaches only once the previous store has read it

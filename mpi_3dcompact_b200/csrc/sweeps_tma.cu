@@ -130,9 +130,25 @@ int launch_tma_yz_kind(const Grid3 &g, const LineOpDev<float> &op, const SweepBa
     return MC3D_ERR_CONFIG;
 }
 
+// a CTA per tile, with one tile and the chain states
+template <int KIND, int H, int L, int E>
+int launch_tma_x_epi(const Grid3 &g, const LineOpDev<float> &op, const TmaMaps &maps, int nf, int py, int pz,
+                     cudaStream_t st) {
+    const int S = op.N / L;
+    const size_t smem = 1024 + (size_t)(op.N / TMA_BOX) * 4096 + (size_t)reg_chain_elems(S) * sizeof(float);
+    auto kern = sweep_tma_x_kernel<KIND, H, L, E>;
+    static KernelLaunchState ls;
+    if (int rc = open_kernel(kern, ls, smem, 0, nullptr)) return rc;
+    kern<<<dim3(tile_count<0>(g), nf), 32 * S, smem, st>>>(g, op, maps, py, pz);
+    MC3D_CUDA_TRY(cudaGetLastError());
+    return MC3D_OK;
+}
+
 template <int KIND, int H, int L, int E>
 int launch_tma_epi(const Grid3 &g, const LineOpDev<float> &op, const TmaMaps &maps, int nf, int py, int pz,
                    cudaStream_t st) {
+    // two tiles of longer lines leave room for one CTA per SM
+    if (op.N > 256) return launch_tma_x_epi<KIND, H, L, E>(g, op, maps, nf, py, pz, st);
     // input and output tiles, chain states; persistent CTAs, as many as fit
     const int S = op.N / L;
     const size_t smem = 1024 + 2 * (size_t)(op.N / TMA_BOX) * 4096 + (size_t)reg_chain_elems(S) * sizeof(float);
@@ -152,6 +168,7 @@ int launch_tma_kind(const Grid3 &g, const LineOpDev<float> &op, const TmaMaps &m
     if (epi == EPI_STORE) return launch_tma_epi<KIND, H, 64, EPI_STORE>(g, op, maps, nf, py, pz, st);
     if constexpr (H <= 3) {
         if (epi == EPI_STORE_NEG) return launch_tma_epi<KIND, H, 64, EPI_STORE_NEG>(g, op, maps, nf, py, pz, st);
+        if (epi == EPI_SUB) return launch_tma_x_epi<KIND, H, 64, EPI_SUB>(g, op, maps, nf, py, pz, st);
     }
     return MC3D_ERR_CONFIG;
 }
@@ -165,11 +182,27 @@ int launch_sweep_tma_x(const Grid3 &g, const LineOpDev<float> &op, const SweepBa
         return e && e[0] == '1';
     }();
     if (disabled) return MC3D_ERR_CONFIG;
-    // stores and negated stores (the latter without pass-through lines) of
-    // lines up to 256 values in 64-row segments
-    if (!(epi == EPI_STORE || (epi == EPI_STORE_NEG && !px && !py && !pz))) return MC3D_ERR_CONFIG;
-    if (op.L != 64 || op.N % TMA_BOX != 0 || op.N > 256 || op.N != g.Nx) return MC3D_ERR_CONFIG;
-    if (b.nf < 1 || b.nf > TMA_MAXF) return MC3D_ERR_CONFIG;
+    // stores, and negated stores and accumulation without pass-through lines, of
+    // lines in 64-row segments (up to 1024 values: 16 segments)
+    if (!(epi == EPI_STORE || ((epi == EPI_STORE_NEG || epi == EPI_SUB) && !px && !py && !pz))) return MC3D_ERR_CONFIG;
+    if (op.L != 64 || op.N % TMA_BOX != 0 || op.N > 1024 || op.N != g.Nx) return MC3D_ERR_CONFIG;
+    if (op.keep && (op.N > 256 || epi == EPI_SUB || b.nf > TMA_MAXF)) return MC3D_ERR_CONFIG;
+    if (b.nf < 1) return MC3D_ERR_CONFIG;
+    if (b.nf > TMA_MAXF) {   // one launch per TMA_MAXF fields, all of them through TMA or none
+        for (int f = 0; f < b.nf; f++)
+            if ((((uintptr_t)b.in[f] | (uintptr_t)b.out[f]) & 15) != 0) return MC3D_ERR_CONFIG;
+        for (int f0 = 0; f0 < b.nf; f0 += TMA_MAXF) {
+            SweepBatch<float> part{};
+            part.nf = std::min(TMA_MAXF, b.nf - f0);
+            for (int f = 0; f < part.nf; f++) {
+                part.in[f] = b.in[f0 + f];
+                part.out[f] = b.out[f0 + f];
+            }
+            const int rc = launch_sweep_tma_x(g, op, part, epi, px, py, pz, st);
+            if (rc != MC3D_OK) return f0 && rc == MC3D_ERR_CONFIG ? fail(rc, "no tensor map for the x lines") : rc;
+        }
+        return MC3D_OK;
+    }
     const long long lines = (long long)g.Ny * g.Nz;
     TmaMaps maps;
     for (int f = 0; f < b.nf; f++)
