@@ -459,11 +459,15 @@ int mc3d_solver_set_timing(mc3d_solver s, int enable);
 const char *mc3d_solver_timing_report(mc3d_solver s);
 
 /* Number of bounded waits on `device` that gave up: line-solve CTAs whose TMA
- * tile load did not arrive (they skipped their tile) plus learned-closure
- * warpgroups whose tensor-core MMAs did not complete (they stopped); the
- * results of those launches are invalid. mc3d_solver_info and
+ * tile load or bulk copy did not arrive (they skipped their tile) plus
+ * learned-closure warpgroups whose tensor-core MMAs did not complete (they
+ * stopped); the results of those launches are invalid. mc3d_solver_info and
  * mc3d_solver_get_conserved return MC3D_ERR_TIMEOUT when it is nonzero. */
 int mc3d_tma_wait_timeouts(int device, int *count);
+/* Sets the count of one family of waits (0: TMA tile loads, 1: bulk copies of
+ * x lines, 2: closure MMAs): to 0 once the application has dealt with a
+ * reported time-out, or to another value to rehearse one. */
+int mc3d_set_wait_timeouts(int device, int family, int count);
 
 /* ---- SGS models on their own (AbstractSGS, src/AbstractSGS.hpp:10-42) ----
  * A GPU VremanSGS / DSMSGS (src/VremanSGS.hpp:13-41, src/DSMSGS.hpp:20-118)

@@ -216,8 +216,7 @@ def write_dump(path, time_step, time, fields):
 
 
 def tma_wait_timeouts(device=0):
-    """Line-solve CTAs on `device` whose TMA tile load gave up waiting (0 in a
-    healthy run)."""
+    """Bounded device waits on `device` that gave up (0 in a healthy run)."""
     n = C.c_int()
     N.check(N.host_lib().mc3d_tma_wait_timeouts(int(device), C.byref(n)))
     return n.value

@@ -599,3 +599,44 @@ extern "C" int mc3d_hit_randvec(int *state, double *r, long long n, double *out)
     state[2] = (int)ix3;
     return MC3D_OK;
 }
+
+// ---------------------------------------------------------------------------
+// bounded device waits that gave up
+// ---------------------------------------------------------------------------
+namespace mc3d {
+static int wait_counter(int family, int **dev) {
+    switch (family) {
+        case WAIT_TMA: return wait_counter_tma(dev);
+        case WAIT_RAG_X: return wait_counter_rag_x(dev);
+        case WAIT_MLP: return wait_counter_mlp(dev);
+    }
+    return fail(MC3D_ERR_ARG, "unknown family of waits");
+}
+
+int wait_timeouts(int count[WAIT_FAMILIES]) {
+    for (int k = 0; k < WAIT_FAMILIES; k++) {
+        int *dev = nullptr;
+        if (int rc = wait_counter(k, &dev)) return rc;
+        MC3D_CUDA_TRY(cudaMemcpy(&count[k], dev, sizeof(int), cudaMemcpyDeviceToHost));
+    }
+    return MC3D_OK;
+}
+}  // namespace mc3d
+
+extern "C" int mc3d_tma_wait_timeouts(int device, int *count) {
+    if (!count) return fail(MC3D_ERR_ARG, "null argument");
+    MC3D_CUDA_TRY(cudaSetDevice(device));
+    int n[WAIT_FAMILIES];
+    if (int rc = wait_timeouts(n)) return rc;
+    *count = 0;
+    for (int c : n) *count += c;
+    return MC3D_OK;
+}
+
+extern "C" int mc3d_set_wait_timeouts(int device, int family, int count) {
+    MC3D_CUDA_TRY(cudaSetDevice(device));
+    int *dev = nullptr;
+    if (int rc = wait_counter(family, &dev)) return rc;
+    MC3D_CUDA_TRY(cudaMemcpy(dev, &count, sizeof(int), cudaMemcpyHostToDevice));
+    return MC3D_OK;
+}

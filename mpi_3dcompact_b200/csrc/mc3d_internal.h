@@ -327,8 +327,6 @@ int mlp_train_step(MlpDev &m, const float *x, const float *y, int n, float lr, f
                    double *loss, cudaStream_t st);
 // tensor-core inference of raw features x [n][9] -> raw outputs [n][2] (sgs_mlp.cu)
 int mlp_infer_bf16(const MlpDev &m, const float *x, int n, float *out, cudaStream_t st);
-// MMA completions that did not arrive within the wait limit (tensor-core inference)
-int mlp_wait_timeouts(int *count);
 const MlpDev *mlp_dev(mc3d_mlp m);
 // fused closure in the time step: d[12] the xi-derivatives of U, V, W, T
 template <typename R>
@@ -487,9 +485,16 @@ int launch_turb_sums(const Grid3 &g, const R *const prim[5], const R *const d[12
 int launch_wall_span_average(const Grid3 &g, const double *const q[5], double *out, cudaStream_t st);
 int launch_wake_strip(const Grid3 &g, const double *const q[5], int i, int j, double *out, cudaStream_t st);
 
-// CTAs of the TMA-staged line solves on the current device whose tile load
-// did not arrive within the wait limit (their results are invalid)
-int tma_wait_timeouts(int *count);
+// Bounded device waits that gave up, counted by family of kernels (the results
+// of those launches are invalid): tile loads of the TMA-staged line solves, bulk
+// copies of the ragged x lines, MMA completions of the learned closure. One
+// counter a family and device, each in the translation unit of its kernels.
+enum { WAIT_TMA, WAIT_RAG_X, WAIT_MLP, WAIT_FAMILIES };
+int wait_counter_tma(int **dev);
+int wait_counter_rag_x(int **dev);
+int wait_counter_mlp(int **dev);
+// every family's count on the current device (capi.cpp)
+int wait_timeouts(int count[WAIT_FAMILIES]);
 
 // ---- checkpoint files (checkpoint.cpp) ----------------------------------------
 int write_solution_dump(const char *path, int time_step, double time, int Nx, int Ny, int Nz,

@@ -292,8 +292,8 @@ int mlp_infer_bf16(const MlpDev &m, const float *x, int n, float *out, cudaStrea
     return MC3D_OK;
 }
 
-int mlp_wait_timeouts(int *count) {
-    MC3D_CUDA_TRY(cudaMemcpyFromSymbol(count, g_mlp_wait_timeouts, sizeof(int)));
+int wait_counter_mlp(int **dev) {
+    MC3D_CUDA_TRY(cudaGetSymbolAddress((void **)dev, g_mlp_wait_timeouts));
     return MC3D_OK;
 }
 

@@ -766,16 +766,15 @@ static int stage_post(mc3d_solver s) {
     return face_poststep<R>(s);
 }
 
-// MC3D_ERR_TIMEOUT when a line-solve tile load or a tensor-core MMA of the
-// learned closure gave up waiting on this device
-static int tma_timeouts_failed(mc3d_solver s) {
-    (void)s;
-    int n = 0, nm = 0;
-    if (int rc = tma_wait_timeouts(&n)) return rc;
-    if (n) return fail(MC3D_ERR_TIMEOUT, "a line-solve tile load did not arrive within the wait limit");
-    if (int rc = mlp_wait_timeouts(&nm)) return rc;
-    return nm ? fail(MC3D_ERR_TIMEOUT, "a tensor-core MMA of the learned closure did not complete within the wait limit")
-              : MC3D_OK;
+// MC3D_ERR_TIMEOUT when a bounded wait of any kernel gave up on this device
+static int wait_timeouts_failed() {
+    int n[WAIT_FAMILIES];
+    if (int rc = wait_timeouts(n)) return rc;
+    if (n[WAIT_TMA] || n[WAIT_RAG_X])
+        return fail(MC3D_ERR_TIMEOUT, "a line-solve tile load did not arrive within the wait limit");
+    return n[WAIT_MLP] ? fail(MC3D_ERR_TIMEOUT,
+                              "a tensor-core MMA of the learned closure did not complete within the wait limit")
+                       : MC3D_OK;
 }
 
 // bit f: face f is a SPONGE
@@ -1988,7 +1987,7 @@ int mc3d_solver_get_conserved(mc3d_solver s, double *rho, double *rhoU, double *
     TimeState t;
     MC3D_CUDA_TRY(cudaMemcpy(&t, s->ts, sizeof(t), cudaMemcpyDeviceToHost));
     if (t.nonfinite) return fail(MC3D_ERR_NONFINITE, "the state became non-finite");
-    if (int rc_tma = tma_timeouts_failed(s)) return rc_tma;
+    if (int rc_wait = wait_timeouts_failed()) return rc_wait;
     return MC3D_OK;
 }
 
@@ -2207,7 +2206,7 @@ int mc3d_solver_info(mc3d_solver s, int *time_step, double *time, double *dt, lo
     if (dt) *dt = t.dt;
     if (stages) *stages = s->stages;
     if (t.nonfinite) return fail(MC3D_ERR_NONFINITE, "the state became non-finite");
-    if (int rc_tma = tma_timeouts_failed(s)) return rc_tma;
+    if (int rc_wait = wait_timeouts_failed()) return rc_wait;
     return MC3D_OK;
 }
 

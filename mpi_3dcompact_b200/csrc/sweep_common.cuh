@@ -105,9 +105,6 @@ template <int DIR, typename R>
 int launch_sweep_rag(const Grid3 &g, const LineOpDev<R> &op, const SweepBatch<R> &b, int epi,
                      const RhsFinalArgs<R> &rf, int px, int py, int pz, cudaStream_t st);
 
-// CTAs of the ragged x kernel whose wait for a bulk copy gave up
-int x_wait_timeouts_rag(int *count);
-
 // FP32 x-line solves staged through shared memory by TMA (sweep_tma.cuh,
 // sweeps_tma.cu);
 // MC3D_ERR_CONFIG, without recording an error, when the case is not covered

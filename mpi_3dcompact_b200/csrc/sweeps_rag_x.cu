@@ -6,8 +6,8 @@ template int launch_sweep_rag<0, float>(const Grid3 &, const LineOpDev<float> &,
                                          const RhsFinalArgs<float> &, int, int, int, cudaStream_t);
 template int launch_sweep_rag<0, double>(const Grid3 &, const LineOpDev<double> &, const SweepBatch<double> &, int,
                                           const RhsFinalArgs<double> &, int, int, int, cudaStream_t);
-int x_wait_timeouts_rag(int *count) {
-    MC3D_CUDA_TRY(cudaMemcpyFromSymbol(count, g_bulk_wait_timeouts, sizeof(int)));
+int wait_counter_rag_x(int **dev) {
+    MC3D_CUDA_TRY(cudaGetSymbolAddress((void **)dev, g_bulk_wait_timeouts));
     return MC3D_OK;
 }
 }  // namespace mc3d

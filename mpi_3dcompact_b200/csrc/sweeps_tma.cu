@@ -264,20 +264,9 @@ int launch_sweep_tma_yz(int dir, const Grid3 &g, const LineOpDev<float> &op, con
     return MC3D_ERR_CONFIG;
 }
 
-int tma_wait_timeouts(int *count) {
-    MC3D_CUDA_TRY(cudaMemcpyFromSymbol(count, g_tma_wait_timeouts, sizeof(int)));
+int wait_counter_tma(int **dev) {
+    MC3D_CUDA_TRY(cudaGetSymbolAddress((void **)dev, g_tma_wait_timeouts));
     return MC3D_OK;
 }
 
 }  // namespace mc3d
-
-extern "C" int mc3d_tma_wait_timeouts(int device, int *count) {
-    if (!count) return mc3d::fail(MC3D_ERR_ARG, "null argument");
-    MC3D_CUDA_TRY(cudaSetDevice(device));
-    int n[3] = {0, 0, 0};
-    if (int rc = mc3d::tma_wait_timeouts(&n[0])) return rc;
-    if (int rc = mc3d::mlp_wait_timeouts(&n[1])) return rc;
-    if (int rc = mc3d::x_wait_timeouts_rag(&n[2])) return rc;
-    *count = n[0] + n[1] + n[2];
-    return MC3D_OK;
-}

@@ -24,3 +24,12 @@ def pytest_collection_modifyitems(config, items):
     for it in items:
         if "gpu" in it.keywords:
             it.add_marker(skip)
+
+
+@pytest.fixture(autouse=True)
+def no_wait_gave_up(request):
+    """After every GPU test: no bounded device wait gave up during it."""
+    yield
+    if "gpu" in request.keywords:
+        import mpi_3dcompact_b200 as m
+        assert m.tma_wait_timeouts(0) == 0

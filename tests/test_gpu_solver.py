@@ -225,6 +225,34 @@ def test_fp32bulk_tma_line_solves_follow_fp64():
     assert m.tma_wait_timeouts(0) == 0
 
 
+def test_every_wait_that_gave_up_reaches_the_solver():
+    """A count in any family of bounded waits (TMA tiles, bulk-copied ragged x
+    lines, closure MMAs), set on the host as a kernel that gave up would leave
+    it: the public total shows it, and info() and conserved() raise
+    MC3D_ERR_TIMEOUT until the count is cleared."""
+    from mpi_3dcompact_b200 import _native as N
+    lib = N.host_lib()
+    s = m.CurvilinearCSolver(m.Options(grid=(13, 12, 11)))
+    s.set_box_metrics(2.0 * math.pi)
+    rng = np.random.default_rng(3)
+    s.set_initial_conditions(*[1.0 + 0.01 * rng.standard_normal((11, 12, 13)) for _ in range(5)])
+    s.step(1)
+    for family in range(3):
+        try:
+            N.check(lib.mc3d_set_wait_timeouts(0, family, 2))
+            assert m.tma_wait_timeouts(0) == 2, family
+            for call in (s.info, s.conserved):
+                with pytest.raises(N.Mc3dError) as e:
+                    call()
+                assert e.value.code == 5, (family, str(e.value))   # MC3D_ERR_TIMEOUT
+        finally:
+            N.check(lib.mc3d_set_wait_timeouts(0, family, 0))
+        assert m.tma_wait_timeouts(0) == 0
+        s.info()
+        s.conserved()
+    assert lib.mc3d_set_wait_timeouts(0, 3, 1) == 6   # MC3D_ERR_ARG
+
+
 def test_ten_steps_match_reference_solver():
     """The bench's scheme for 10 time steps (55 LSLDDRK4 stages) on 64 x 24 x 16:
     FP64 within 1e-12 relative of the reference solver per conserved field,
