@@ -106,13 +106,28 @@ struct mc3d_solver_s {
 
 namespace mc3d {
 
-// Whether a solver's lines may take the ragged segmented solve. Not with the
-// dynamic model in FP32: its coefficient is a ratio of averages that magnifies
-// the operators' rounding (another order of the same FP32 sums moves the
-// spanwise momentum of an O-grid by 2e-5 relative within two steps, the distance
-// of either from FP64 being 4e-5), so those solvers keep the whole-line order.
-static bool ragged_lines(int les_model, int precision) {
-    return !(les_model == MC3D_DSM && precision != MC3D_FP64);
+// Whether a solver's (or SGS object's) lines may take the ragged segmented solve
+// and the long-line TMA kernels. Not in FP32 where the dynamic model can run:
+// its coefficient is a ratio of averages that magnifies the operators' rounding
+// (another order of the same FP32 sums moves the spanwise momentum of an O-grid
+// by 2e-5 relative within two steps, the distance of either from FP64 being
+// 4e-5), so every such run keeps one order of sums, the whole-line one: the DSM
+// solver, the standalone DSM object, and the learned closure's solver unless no
+// stage of it can fall back to DSM.
+static bool ragged_lines(const mc3d_config &c) {
+    const bool dynamic = c.les_model == MC3D_DSM ||
+                         (c.les_model == MC3D_MLPSGS && !c.lean_storage && c.mlp_fallback_frac < 1.0);
+    return !(dynamic && c.precision != MC3D_FP64);
+}
+
+// The dynamic model's test filter along d: DSMTESTFILTER 1 -> Pade, 2 -> explicit
+// (src/DSMSGS.hpp:57-67)
+static int upload_test_filter(mc3d_solver s, int d) {
+    const mc3d_config &c = s->cfg;
+    const int N[3] = {c.Nx, c.Ny, c.Nz};
+    return upload_line_op(build_testfilter_op(c.dsm_test_filter == 1 ? MC3D_TESTFILTER_PADE : MC3D_TESTFILTER_EXP,
+                                              c.bc_type[d], N[d]),
+                          c.precision, s->top[d], ragged_lines(c));
 }
 
 // Blocks up to this many points run their gradient sweeps side by side
@@ -1026,15 +1041,10 @@ int mc3d_solver_create(const mc3d_config *cfg, int device, mc3d_solver *out) {
             LineOpHost dh = build_deriv_op(c.fd_type[d], c.bc_type[d], N[d], s->dxi[d]);
             LineOpHost fh = build_filter_op(c.filter_type, c.alphaF, c.bc_type[d], N[d]);
             LineOpHost vh = build_filter_op(MC3D_COMPACT10, -0.49, c.bc_type[d], N[d]);
-            if ((rc = upload_line_op(dh, c.precision, s->dop[d], ragged_lines(c.les_model, c.precision)))) break;
-            if ((rc = upload_line_op(fh, c.precision, s->fop[d], ragged_lines(c.les_model, c.precision)))) break;
-            if ((rc = upload_line_op(vh, c.precision, s->vop[d], ragged_lines(c.les_model, c.precision)))) break;
-            if (c.les_model == MC3D_DSM || c.les_model == MC3D_MLPSGS) {
-                // DSMTESTFILTER 1 -> Pade, 2 -> explicit (src/DSMSGS.hpp:57-67)
-                LineOpHost th = build_testfilter_op(c.dsm_test_filter == 1 ? MC3D_TESTFILTER_PADE : MC3D_TESTFILTER_EXP,
-                                                    c.bc_type[d], N[d]);
-                if ((rc = upload_line_op(th, c.precision, s->top[d], ragged_lines(c.les_model, c.precision)))) break;
-            }
+            if ((rc = upload_line_op(dh, c.precision, s->dop[d], ragged_lines(c)))) break;
+            if ((rc = upload_line_op(fh, c.precision, s->fop[d], ragged_lines(c)))) break;
+            if ((rc = upload_line_op(vh, c.precision, s->vop[d], ragged_lines(c)))) break;
+            if ((c.les_model == MC3D_DSM || c.les_model == MC3D_MLPSGS) && (rc = upload_test_filter(s, d))) break;
         }
     } catch (const std::exception &ex) {
         rc = fail(MC3D_ERR_CONFIG, ex.what());
@@ -1331,7 +1341,7 @@ static int compute_metrics(mc3d_solver s, const double *hx, const double *hy, co
     try {
         for (int d = 0; d < 3 && !rc; d++) {
             LineOpHost h = build_deriv_op(s->cfg.fd_type[d], s->cfg.bc_type[d], Ns[d], s->dxi[d]);
-            if ((rc = upload_line_op(h, MC3D_FP64, md[d].deriv, ragged_lines(s->cfg.les_model, s->prec)))) break;
+            if ((rc = upload_line_op(h, MC3D_FP64, md[d].deriv, ragged_lines(s->cfg)))) break;
             md[d].periodic = s->cfg.bc_type[d] == MC3D_PERIODIC_SOLVE;
             md[d].cd2 = s->cfg.fd_type[d] == MC3D_CD2;
             md[d].H = h.H;
@@ -1343,7 +1353,7 @@ static int compute_metrics(mc3d_solver s, const double *hx, const double *hy, co
                 sv.st[sv.H] = 1.0;
                 sv.deriv = false;
                 sv.inv_dh = 1.0;
-                rc = upload_line_op(sv, MC3D_FP64, md[d].solve, ragged_lines(s->cfg.les_model, s->prec));
+                rc = upload_line_op(sv, MC3D_FP64, md[d].solve, ragged_lines(s->cfg));
             }
         }
     } catch (const std::exception &e) {
@@ -2354,10 +2364,7 @@ int mc3d_sgs_create(int model, int averaging, int test_filter, int use_taukk, in
                 // VremanSGS averages with Compact10 filters of alpha -0.49 (src/VremanSGS.hpp:38-40)
                 rc = upload_line_op(build_filter_op(MC3D_COMPACT10, -0.49, bc_types[d], N[d]), precision, s->vop[d]);
             } else {
-                // DSMTESTFILTER 1 -> Pade, 2 -> explicit (src/DSMSGS.hpp:57-67)
-                rc = upload_line_op(build_testfilter_op(test_filter == 1 ? MC3D_TESTFILTER_PADE : MC3D_TESTFILTER_EXP,
-                                                        bc_types[d], N[d]),
-                                    precision, s->top[d]);
+                rc = upload_test_filter(s, d);
             }
         }
     } catch (const std::exception &ex) {

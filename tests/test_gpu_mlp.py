@@ -334,3 +334,72 @@ def test_sgs_object_with_the_closure_reports_misuse_and_range():
     assert count.value == n ** 3
     assert torch.isfinite(mu).all() and torch.isfinite(ks).all()
     N.check(lib.mc3d_sgs_destroy(o))
+
+
+def test_forced_fallback_equals_the_dsm_solver_on_ragged_lines():
+    """FP32 on lines of 75, 34 and 40 points: a closure whose training range no
+    state can lie in sends every stage to DSM, and the state after two steps
+    equals a DSM solver's bit for bit (one order of the operators' sums wherever
+    the dynamic model can run, whose coefficient magnifies their rounding)."""
+    N = (75, 34, 40)
+    z, y, x = np.meshgrid(*[2 * math.pi * np.arange(n) / n for n in N[::-1]], indexing="ij")
+    ic = [1.0 + 0.02 * np.cos(x + y), 0.3 * np.sin(x) * np.cos(y + z), 0.2 * np.cos(2 * x - z) + 0.1 * np.sin(3 * y),
+          0.25 * np.sin(y) * np.cos(z) + 0.1 * np.cos(4 * x), 1.0 / 1.4 + 0.01 * np.sin(x - z)]
+    net = m.MLPClosure(seed=6)
+    one = np.ones(9, np.float32)
+    net.set_normalization(0 * one, one, 1e30 * one, 1e31 * one, np.zeros(2, np.float32), np.ones(2, np.float32))
+    out = {}
+    for les in ("DSM", "MLP"):
+        s = m.CurvilinearCSolver(m.Options(grid=N, fd="PADE6", filter="COMPACT10", alphaF=0.49, rk="RK4", mu_ref=1e-3,
+                                           les=les, les_avg="GLOBAL", precision=m.FP32BULK, mlp_fallback_frac=1e-3))
+        s.set_box_metrics(2.0 * math.pi)
+        s.set_initial_conditions(*ic)
+        if les == "MLP":
+            s.set_mlp(net)
+        s.step(2)
+        out[les] = s.conserved()
+        if les == "MLP":
+            assert s.mlp_fallbacks() == 8
+    for i in range(5):
+        assert np.isfinite(out["DSM"][i]).all()
+        assert np.array_equal(out["DSM"][i], out["MLP"][i]), (i, float(np.abs(out["DSM"][i] - out["MLP"][i]).max()))
+
+
+def test_standalone_dsm_object_keeps_the_solvers_order_of_sums():
+    """The standalone FP32 DSM object sums its test filters in the DSM solver's
+    whole-line order. Seen from outside: the filter is translation invariant, and
+    on a 511-point periodic line the whole-line recurrences forget their start
+    (by 0.65 a row) well before row 130, so fields moved by 16 points give the
+    same bits moved by 16 points. Solved in segments of 32 rows they would not:
+    each segment's rows add a response that starts at the segment's edge."""
+    import ctypes as C
+    torch = _torch()
+    from mpi_3dcompact_b200 import _native as N
+    lib = N.host_lib()
+    nz, ny, nx = 12, 16, 511
+    h = C.c_void_p()
+    N.check(lib.mc3d_sgs_create(N.DSM, N.AVG_XI2, 1, 1, nx, ny, nz, (C.c_int * 3)(0, 0, 0),
+                                (C.c_double * 3)(1.0 / nx, 1.0 / ny, 1.0 / nz), None, 0.5, m.FP32BULK, 0, C.byref(h)))
+    rng = np.random.default_rng(8)
+    g = [torch.tensor(rng.standard_normal((nz, ny, nx)).astype(np.float32), device="cuda") for _ in range(12)]
+    q = [torch.tensor(2.0 + 0.1 * rng.standard_normal((nz, ny, nx)), device="cuda") for _ in range(5)]
+    T = 1.0 + 0.01 * g[0]
+
+    def vp(ts):
+        return (C.c_void_p * len(ts))(*[t.data_ptr() for t in ts])
+
+    def run(shift):
+        gs, qs = [[torch.roll(t, shift, 2).contiguous() for t in ts] for ts in (g, q)]
+        Ts = torch.roll(T, shift, 2).contiguous()
+        mu, tk, ks = (torch.empty_like(T) for _ in range(3))
+        N.check(lib.mc3d_sgs_calc_mu_taukk(h, vp(gs[:9]), vp(qs), C.c_void_p(mu.data_ptr()), C.c_void_p(tk.data_ptr()),
+                                           None))
+        N.check(lib.mc3d_sgs_calc_ksgs(h, vp(gs[9:]), vp(qs), C.c_void_p(Ts.data_ptr()), C.c_void_p(ks.data_ptr()),
+                                       None))
+        torch.cuda.synchronize()
+        return [a.cpu().numpy() for a in (mu, tk, ks)]
+    a, b = run(0), run(16)
+    N.check(lib.mc3d_sgs_destroy(h))
+    for name, u, v in zip(("mu_sgs", "taukk", "k_sgs"), a, b):
+        assert np.isfinite(u).all() and np.abs(u).max() > 0, name
+        assert np.array_equal(u[:, :, 130:380], v[:, :, 146:396]), name
