@@ -173,6 +173,24 @@ int launch_tma_kind(const Grid3 &g, const LineOpDev<float> &op, const TmaMaps &m
     return MC3D_ERR_CONFIG;
 }
 
+int launch_tma_x_op(const Grid3 &g, const LineOpDev<float> &op, const TmaMaps &maps, int nf, int epi, int py, int pz,
+                    cudaStream_t st) {
+#define MC3D_TCASE(K, HH) \
+    if (op.kind == K && op.H == HH) return launch_tma_kind<K, HH>(g, op, maps, nf, epi, py, pz, st);
+    MC3D_TCASE(K_TRI_PER, 2)
+    MC3D_TCASE(K_TRI_DIR, 2)
+    MC3D_TCASE(K_PEN_PER, 3)
+    MC3D_TCASE(K_PEN_DIR, 3)
+    MC3D_TCASE(K_TRI_PER, 4)
+    MC3D_TCASE(K_TRI_DIR, 4)
+    MC3D_TCASE(K_TRI_PER, 5)
+    MC3D_TCASE(K_TRI_DIR, 5)
+    MC3D_TCASE(K_PEN_PER, 5)
+    MC3D_TCASE(K_PEN_DIR, 5)
+#undef MC3D_TCASE
+    return MC3D_ERR_CONFIG;
+}
+
 }  // namespace
 
 int launch_sweep_tma_x(const Grid3 &g, const LineOpDev<float> &op, const SweepBatch<float> &b, int epi, int px,
@@ -187,38 +205,25 @@ int launch_sweep_tma_x(const Grid3 &g, const LineOpDev<float> &op, const SweepBa
     if (!(epi == EPI_STORE || ((epi == EPI_STORE_NEG || epi == EPI_SUB) && !px && !py && !pz))) return MC3D_ERR_CONFIG;
     if (op.L != 64 || op.N % TMA_BOX != 0 || op.N > 1024 || op.N != g.Nx) return MC3D_ERR_CONFIG;
     if (op.keep && (op.N > 256 || epi == EPI_SUB || b.nf > TMA_MAXF)) return MC3D_ERR_CONFIG;
-    if (b.nf < 1) return MC3D_ERR_CONFIG;
-    if (b.nf > TMA_MAXF) {   // one launch per TMA_MAXF fields, all of them through TMA or none
-        for (int f = 0; f < b.nf; f++)
-            if ((((uintptr_t)b.in[f] | (uintptr_t)b.out[f]) & 15) != 0) return MC3D_ERR_CONFIG;
-        for (int f0 = 0; f0 < b.nf; f0 += TMA_MAXF) {
-            SweepBatch<float> part{};
-            part.nf = std::min(TMA_MAXF, b.nf - f0);
-            for (int f = 0; f < part.nf; f++) {
-                part.in[f] = b.in[f0 + f];
-                part.out[f] = b.out[f0 + f];
-            }
-            const int rc = launch_sweep_tma_x(g, op, part, epi, px, py, pz, st);
-            if (rc != MC3D_OK) return f0 && rc == MC3D_ERR_CONFIG ? fail(rc, "no tensor map for the x lines") : rc;
-        }
-        return MC3D_OK;
-    }
+    // one launch per TMA_MAXF fields. Every launch's maps are made before the
+    // first launch: nothing has run yet when the batch turns out not to be covered
+    // and goes to the register kernel as a whole.
+    constexpr int MAXL = 2;
+    if (b.nf < 1 || b.nf > MAXL * TMA_MAXF) return MC3D_ERR_CONFIG;
     const long long lines = (long long)g.Ny * g.Nz;
-    TmaMaps maps;
-    for (int f = 0; f < b.nf; f++)
-        if (!tensor_map_x(b.in[f], g.Nx, lines, &maps.in[f]) || !tensor_map_x(b.out[f], g.Nx, lines, &maps.out[f]))
+    TmaMaps maps[MAXL];
+    for (int f = 0; f < b.nf; f++) {
+        TmaMaps &m = maps[f / TMA_MAXF];
+        const int k = f % TMA_MAXF;
+        if (!tensor_map_x(b.in[f], g.Nx, lines, &m.in[k]) || !tensor_map_x(b.out[f], g.Nx, lines, &m.out[k]))
             return MC3D_ERR_CONFIG;
-    if (op.kind == K_TRI_PER && op.H == 2) return launch_tma_kind<K_TRI_PER, 2>(g, op, maps, b.nf, epi, py, pz, st);
-    if (op.kind == K_TRI_DIR && op.H == 2) return launch_tma_kind<K_TRI_DIR, 2>(g, op, maps, b.nf, epi, py, pz, st);
-    if (op.kind == K_PEN_PER && op.H == 3) return launch_tma_kind<K_PEN_PER, 3>(g, op, maps, b.nf, epi, py, pz, st);
-    if (op.kind == K_PEN_DIR && op.H == 3) return launch_tma_kind<K_PEN_DIR, 3>(g, op, maps, b.nf, epi, py, pz, st);
-    if (op.kind == K_TRI_PER && op.H == 4) return launch_tma_kind<K_TRI_PER, 4>(g, op, maps, b.nf, epi, py, pz, st);
-    if (op.kind == K_TRI_DIR && op.H == 4) return launch_tma_kind<K_TRI_DIR, 4>(g, op, maps, b.nf, epi, py, pz, st);
-    if (op.kind == K_TRI_PER && op.H == 5) return launch_tma_kind<K_TRI_PER, 5>(g, op, maps, b.nf, epi, py, pz, st);
-    if (op.kind == K_TRI_DIR && op.H == 5) return launch_tma_kind<K_TRI_DIR, 5>(g, op, maps, b.nf, epi, py, pz, st);
-    if (op.kind == K_PEN_PER && op.H == 5) return launch_tma_kind<K_PEN_PER, 5>(g, op, maps, b.nf, epi, py, pz, st);
-    if (op.kind == K_PEN_DIR && op.H == 5) return launch_tma_kind<K_PEN_DIR, 5>(g, op, maps, b.nf, epi, py, pz, st);
-    return MC3D_ERR_CONFIG;
+    }
+    for (int f0 = 0; f0 < b.nf; f0 += TMA_MAXF) {
+        // (MC3D_ERR_CONFIG: an operator or operation without a kernel, so from the first launch or none)
+        const int nf = std::min(TMA_MAXF, b.nf - f0);
+        if (int rc = launch_tma_x_op(g, op, maps[f0 / TMA_MAXF], nf, epi, py, pz, st)) return rc;
+    }
+    return MC3D_OK;
 }
 
 int launch_sweep_tma_yz(int dir, const Grid3 &g, const LineOpDev<float> &op, const SweepBatch<float> &b, int epi,

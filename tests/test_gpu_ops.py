@@ -89,6 +89,35 @@ def test_batched_fields_and_large_lines(prec):
             assert H.rel_max(y.double().cpu().numpy(), ref) <= TOL[prec]
 
 
+@pytest.mark.parametrize("nf", [8, 9, 16])
+@pytest.mark.parametrize("n", [256, 320, 512])
+def test_large_batches_of_fp32_x_lines(n, nf):
+    """Batches of eight fields and above (two launches of TMA-staged lines, with
+    one and two tiles a CTA) equal one-field calls bit for bit; with the last
+    field on an odd address the batch goes to the register kernel as a whole and
+    agrees to FP32 rounding."""
+    torch = _torch()
+    shape = (5, 13, n)
+    g = torch.Generator(device="cuda").manual_seed(n + nf)
+    xs = [torch.randn(shape, device="cuda", generator=g) for _ in range(nf)]
+    off = torch.empty(xs[-1].numel() + 1, device="cuda")[1:].view(shape)
+    off.copy_(xs[-1])
+    bcs = [m.PERIODIC_SOLVE] * 3
+    for op in ("PADE6", "PENTA10", "COMPACT8", "COMPACT10", "TESTPADE"):
+        o = _make(op, 0, bcs, shape, m.FP32BULK)
+        one, many = (o.filterField, o.filterFields) if _is_filter(op) else (o.calc1stDerivField, o.calc1stDerivFields)
+        single = [torch.empty_like(x) for x in xs]
+        for x, y in zip(xs, single):
+            one(x, y)
+        ys = [torch.empty_like(x) for x in xs]
+        many(xs, ys)
+        for k, (y, r) in enumerate(zip(ys, single)):
+            assert torch.equal(y, r), (op, k)
+        many(xs[:-1] + [off], ys)
+        for k, (y, r) in enumerate(zip(ys, single)):
+            assert H.rel_max(y.double().cpu().numpy(), r.double().cpu().numpy()) <= 2 * TOL[m.FP32BULK], (op, k)
+
+
 def test_operator_errors_are_reported():
     torch = _torch()
     with pytest.raises(m.Mc3dError):
