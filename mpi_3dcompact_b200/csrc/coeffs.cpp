@@ -501,43 +501,22 @@ bool antisymmetric(const LineOpHost &h) {
     return true;
 }
 
-// Segment count and homogeneous responses for the segmented line solve.
+// Homogeneous responses of a line in S segments of L rows (the last may have fewer).
 // tri:   forward  x_n = -m_n x_{n-1}                        from x_{a-1} = 1
 //        backward x_n = -c_n x_{n+1} rw_n                    from x_b = 1
 // penta: forward  B_n = -m2_{n-1} B_{n-2} - m1_n B_{n-1}     from (B_{a-1}, B_{a-2}) = (1,0) | (0,1)
 //        backward x_n = (-f_n x_{n+2} - C_n x_{n+1}) rD_n    from (x_b, x_{b+1}) = (1,0) | (0,1)
-void segment(LineOpHost &h, int precision, bool ragged) {
-    int n = h.N;
-    bool tri = h.kind == K_TRI_PER || h.kind == K_TRI_DIR;
-    bool pen = h.kind == K_PEN_PER || h.kind == K_PEN_DIR;
-    h.S = 1;
-    h.L = 0;
-    h.rag = false;
-    if (!(tri || pen)) return;
-    const int UB = 8;
-    int S = 0;
-    int Lr = reg_segment_len(n, h.kind, precision);
-    int L = 0;
-    if (Lr) {
-        S = n / Lr;
-        h.L = Lr;
-    } else if (int Lg = ragged && !(precision != MC3D_FP64 && h.H <= 3 && !antisymmetric(h))
-                            ? ragged_segment_len(n, h.kind) : 0) {   // (the FP32 solve of H <= 3: derivatives only)
-        h.L = L = Lg;
-        h.rag = true;
-        S = (n + L - 1) / L;
-    } else {
-        for (int cand : {4, 2})
-            if (n % cand == 0 && (n / cand) % UB == 0 && n / cand >= 32 && n / cand >= h.bw) { S = cand; break; }
-    }
-    if (!S) return;
-    h.S = S;
-    if (!L) L = n / S;
+LineSegments responses(const LineOpHost &h, int S, int L, int precision) {
+    const int n = h.N;
+    const bool tri = h.kind == K_TRI_PER || h.kind == K_TRI_DIR;
+    const bool pen = h.kind == K_PEN_PER || h.kind == K_PEN_DIR;
+    LineSegments g;
+    g.S = S;
     auto A = [&](int a, int i) { return h.arr[(size_t)a * n + i]; };
-    h.sfa.assign(n, 0.0);
-    h.sfb.assign(n, 0.0);
-    h.sba.assign(n, 0.0);
-    h.sbb.assign(n, 0.0);
+    g.sfa.assign(n, 0.0);
+    g.sfb.assign(n, 0.0);
+    g.sba.assign(n, 0.0);
+    g.sbb.assign(n, 0.0);
     for (int w = 0; w < S; w++) {
         int a = w * L, b = std::min(a + L, n);
         for (int which = 0; which < (pen ? 2 : 1); which++) {
@@ -547,7 +526,7 @@ void segment(LineOpHost &h, int precision, bool ragged) {
                 double x;
                 if (tri) x = -A(0, i) * p1;
                 else x = -(i >= 1 ? A(1, i - 1) : 0.0) * p2 - A(0, i) * p1;
-                (which == 0 ? h.sfa : h.sfb)[i] = x;
+                (which == 0 ? g.sfa : g.sfb)[i] = x;
                 p2 = p1;
                 p1 = x;
             }
@@ -557,11 +536,59 @@ void segment(LineOpHost &h, int precision, bool ragged) {
                 double x;
                 if (tri) x = (0.0 - A(2, i) * q1) * A(1, i);
                 else x = (0.0 - A(4, i) * q2 - A(3, i) * q1) * A(2, i);
-                (which == 0 ? h.sba : h.sbb)[i] = x;
+                (which == 0 ? g.sba : g.sbb)[i] = x;
                 q2 = q1;
                 q1 = x;
             }
         }
+    }
+    if (S == 1) return g;
+    // responses below 2^-64 (FP64) / 2^-32 (FP32) of their unit start are dropped
+    const double thr = std::ldexp(1.0, precision == MC3D_FP64 ? -64 : -32);
+    for (int w = 0; w < S; w++)
+        for (int r = 0; r < L && w * L + r < n; r++) {
+            int i = w * L + r;
+            if (std::fabs(g.sfa[i]) > thr || std::fabs(g.sfb[i]) > thr) g.kf = std::max(g.kf, r + 1);
+            if (S * L != n && w == S - 1) continue;   // (nothing comes back into the last segment)
+            if (std::fabs(g.sba[i]) > thr || std::fabs(g.sbb[i]) > thr) g.kb = std::max(g.kb, L - r);
+        }
+    return g;
+}
+
+// The segments of the line solves: equal ones of the register-resident or of the
+// shared-memory kernel, and, where the register kernel's length does not divide
+// N, its ragged ones as well (calls that form does not take, such as x lines off
+// a 16-byte boundary, use the equal ones).
+void segment(LineOpHost &h, int precision, bool ragged) {
+    const int n = h.N;
+    h.seg = LineSegments();
+    h.rseg = LineSegments();
+    h.L = 0;
+    h.rag = false;
+    const bool tri = h.kind == K_TRI_PER || h.kind == K_TRI_DIR, pen = h.kind == K_PEN_PER || h.kind == K_PEN_DIR;
+    if (!(tri || pen)) return;
+    const int UB = 8;
+    if (int Lr = reg_segment_len(n, h.kind, precision)) {
+        h.L = Lr;
+        h.seg = responses(h, n / Lr, Lr, precision);
+        return;
+    }
+    // at least 32 rows a segment in FP32 and 48 in FP64, below which the whole-line
+    // kernel is faster (x derivatives of four fields of 96 x 96 lines, whole line /
+    // two segments: FP32 80 points 29 / 21 us; FP64 80 points 32 / 43 us, 112 points
+    // 75 / 45 us)
+    const int rows = precision == MC3D_FP64 ? 48 : 32;
+    for (int S : {4, 2})
+        if (n % S == 0 && (n / S) % UB == 0 && n / S >= rows && n / S >= h.bw) {
+            h.seg = responses(h, S, n / S, precision);
+            break;
+        }
+    if (!ragged || (precision != MC3D_FP64 && h.H <= 3 && !antisymmetric(h)))   // (the FP32 solve of H <= 3: derivatives only)
+        return;
+    if (int Lg = ragged_segment_len(n, h.kind)) {
+        h.L = Lg;
+        h.rag = true;
+        h.rseg = responses(h, (n + Lg - 1) / Lg, Lg, precision);
     }
 }
 
@@ -613,13 +640,15 @@ void fill_dev(const LineOpHost &h, const char *base, const Layout &lo, LineOpDev
     d.head = h.head.empty() ? nullptr : p + lo.head;
     d.tail = h.tail.empty() ? nullptr : p + lo.tail;
     const R *sg = p + lo.seg;
-    d.S = h.rag ? 1 : h.S;   // (the shared-memory kernels take equal segments only)
-    d.seg_kf = h.seg_kf;
-    d.seg_kb = h.seg_kb;
-    d.sfa = h.S > 1 ? sg : nullptr;
-    d.sfb = h.S > 1 ? sg + n : nullptr;
-    d.sba = h.S > 1 ? sg + 2 * n : nullptr;
-    d.sbb = h.S > 1 ? sg + 3 * n : nullptr;
+    d.S = h.seg.S;
+    d.seg_kf = h.seg.kf;
+    d.seg_kb = h.seg.kb;
+    d.rag_kf = h.rseg.kf;
+    d.rag_kb = h.rseg.kb;
+    d.sfa = h.seg.S > 1 ? sg : nullptr;
+    d.sfb = h.seg.S > 1 ? sg + n : nullptr;
+    d.sba = h.seg.S > 1 ? sg + 2 * n : nullptr;
+    d.sbb = h.seg.S > 1 ? sg + 3 * n : nullptr;
     d.L = h.L;
     d.rag = h.rag;
     d.keep = h.keep;
@@ -648,8 +677,8 @@ std::vector<R> flatten(const LineOpHost &h, Layout &lo) {
     lo.tail = v.size();
     for (double x : h.tail) put(x);
     lo.seg = v.size();
-    if (h.S > 1)
-        for (const std::vector<double> *a : {&h.sfa, &h.sfb, &h.sba, &h.sbb})
+    if (h.seg.S > 1)
+        for (const std::vector<double> *a : {&h.seg.sfa, &h.seg.sfb, &h.seg.sba, &h.seg.sbb})
             for (double x : *a) put(x);
     if (h.L) {
         const int n = h.N;
@@ -698,17 +727,18 @@ std::vector<R> flatten(const LineOpHost &h, Layout &lo) {
                 for (int c = 0; c < 4; c++) put(A(5 + c, i));
             pad(4);
         }
+        const LineSegments &sg = h.rag ? h.rseg : h.seg;
         align4();
         lo.sf2 = v.size();
         for (int i = 0; i < n; i++) {
-            put(h.sfa[i]);
-            put(h.sfb[i]);
+            put(sg.sfa[i]);
+            put(sg.sfb[i]);
         }
         align4();
         lo.sb2 = v.size();
         for (int i = 0; i < n; i++) {
-            put(h.sba[i]);
-            put(h.sbb[i]);
+            put(sg.sba[i]);
+            put(sg.sbb[i]);
         }
         pad(2);
         if (h.kind == K_TRI_DIR || h.kind == K_PEN_DIR) {
@@ -749,19 +779,6 @@ int upload_line_op(const LineOpHost &hin, int precision, LineOpBuf &out, bool ra
     analyse(h, precision);
     segment(h, precision, ragged);
     h.keep = !ragged;
-    if (h.S > 1) {
-        // responses below 2^-64 (FP64) / 2^-32 (FP32) of their unit start are dropped
-        const double thr = std::ldexp(1.0, precision == MC3D_FP64 ? -64 : -32);
-        int n = h.N, L = h.rag ? h.L : n / h.S;
-        h.seg_kf = h.seg_kb = 0;
-        for (int w = 0; w < h.S; w++)
-            for (int r = 0; r < L && w * L + r < n; r++) {
-                int i = w * L + r;
-                if (std::fabs(h.sfa[i]) > thr || std::fabs(h.sfb[i]) > thr) h.seg_kf = std::max(h.seg_kf, r + 1);
-                if (h.rag && w == h.S - 1) continue;   // (nothing comes back into the last segment)
-                if (std::fabs(h.sba[i]) > thr || std::fabs(h.sbb[i]) > thr) h.seg_kb = std::max(h.seg_kb, L - r);
-            }
-    }
     out.precision = precision;
     MC3D_CUDA_TRY(cudaGetDevice(&out.device));
     Layout lo;

@@ -68,6 +68,17 @@ inline int open_kernel(K kern, KernelLaunchState &st, size_t smem, int threads, 
 // Line kinds: periodic kinds are even.
 enum LineKind { K_EXPL_PER = 0, K_EXPL_DIR = 1, K_TRI_PER = 2, K_TRI_DIR = 3, K_PEN_PER = 4, K_PEN_DIR = 5 };
 
+// S segments of a line and, per row, the homogeneous responses of its segment's
+// local forward recurrence (to the two incoming eliminated values: sfa, sfb) and
+// backward recurrence (to the two outgoing solution values: sba, sbb); kf / kb:
+// rows from a segment's start / end over which they are above the precision's
+// cut-off.
+struct LineSegments {
+    int S = 1;
+    std::vector<double> sfa, sfb, sba, sbb;
+    int kf = 0, kb = 0;
+};
+
 // Host-side description, all factors in FP64 (computed with the reference's
 // own elimination order so the GPU reproduces its factors exactly).
 struct LineOpHost {
@@ -94,16 +105,11 @@ struct LineOpHost {
     // Rows [corr_lo, corr_hi) where the cyclic correction columns are below
     // 2^-64 (FP64) / 2^-32 (FP32) of their peak, so the correction is skipped.
     int corr_lo = 0, corr_hi = 0;
-    // Segmented solve: S segments of L = N/S rows per line; homogeneous
-    // responses of the local forward (to the two incoming eliminated values)
-    // and backward (to the two outgoing solution values) recurrences, per row.
-    int S = 1;
-    std::vector<double> sfa, sfb, sba, sbb;
-    // rows from a segment's start (kf) / end (kb) over which the forward /
-    // backward responses are above the precision's cut-off (set at upload)
-    int seg_kf = 0, seg_kb = 0;
+    // Segmented solve (set at upload): equal segments, and the register-resident
+    // kernel's where N is no multiple of its segment length
+    LineSegments seg, rseg;
     int L = 0;   // segment length of the register-resident kernel (0: not used)
-    bool rag = false;   // N is no multiple of L: the last segment has fewer rows
+    bool rag = false;   // N is no multiple of L: the last segment (of rseg) has fewer rows
     bool keep = false;  // uploaded without `ragged`: keep the order (and contraction) of the sums
 };
 
@@ -137,16 +143,17 @@ struct LineOpDev {
     const R *z0, *z1, *z2, *z3;   // penta cyclic Woodbury columns
     int stat_lo, stat_hi, corr_lo, corr_hi;
     R stat_c[5];
-    int S;                         // segments per line (1 = whole-line kernel)
+    int S;                         // equal segments per line (1 = whole-line kernel)
     const R *sfa, *sfb, *sba, *sbb;
     int seg_kf, seg_kb;
-    // Register-resident segmented solve (segment length L = N/S rows, 0 when
-    // the line length does not suit it). Row-interleaved copies of the
+    int rag_kf, rag_kb;            // the same for the ragged segments
+    // Register-resident segmented solve (segments of L rows, 0 when the line
+    // length does not suit it). Row-interleaved copies of the
     // factors so one vector load fetches a row's coefficients:
     //   pf  [N][2]  forward  (m1_n, m2_{n-1}) | tri (m_n, 0); zero where unused
     //   pb  [N][4]  backward (C_n, f_n, rD_n, 0) | tri (c_n, 0, rw_n, 0)
     //   pz  [N][4]  penta cyclic columns (z0..z3)_n
-    //   sf2 [N][2]  (sfa, sfb)_n,  sb2 [N][2]  (sba, sbb)_n
+    //   sf2 [N][2]  (sfa, sfb)_n,  sb2 [N][2]  (sba, sbb)_n (of the ragged segments when rag)
     //   hp, tp [H][MC3D_BWMAX]  Dirichlet boundary rows, zero padded (head on
     //   phi[0..BWMAX-1], tail right-aligned on phi[N-BWMAX..N-1])
     int L;

@@ -348,7 +348,7 @@ __device__ __forceinline__ void reg_solve(const LineOpDev<R> &op, const R (&v)[L
 
     // ---- forward fold: propagate the incoming state through the first kf rows ----
     if (seg > 0) {
-        const int kf = op.seg_kf;
+        const int kf = RAG ? op.rag_kf : op.seg_kf;
 #pragma unroll
         for (int blk = 0; blk < NB; blk++) {
             if (blk * UB < kf) {
@@ -505,7 +505,7 @@ __device__ __forceinline__ void reg_solve(const LineOpDev<R> &op, const R (&v)[L
 
     // ---- backward fold: propagate the incoming state up through the last kb rows ----
     if (seg < S - 1) {
-        const int kb = op.seg_kb;
+        const int kb = RAG ? op.rag_kb : op.seg_kb;
 #pragma unroll
         for (int blk = NB - 1; blk >= 0; blk--) {
             if ((blk + 1) * UB > L - kb) {

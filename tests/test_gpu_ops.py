@@ -245,6 +245,42 @@ def test_ragged_lines_vs_oracle(n, bc, prec):
 
 
 @pytest.mark.parametrize("prec", [m.FP64, m.FP32BULK])
+@pytest.mark.parametrize("bc", [m.PERIODIC_SOLVE, m.DIRICHLET_SOLVE])
+@pytest.mark.parametrize("n", [75, 80, 144, 496])
+def test_ragged_x_lines_off_a_16_byte_boundary(n, bc, prec):
+    """x lines whose input, output or both start one element past a 16-byte
+    boundary: the ragged solve's bulk copies cannot take them, so they go to the
+    whole-line kernel (75, and 80 in FP64) or to the one of two equal segments."""
+    torch = _torch()
+    from oracle import mc3d_oracle as O
+    rng = np.random.default_rng(n + bc)
+    dt = torch.float64 if prec == m.FP64 else torch.float32
+    shape = (3, 13, n)
+    f = rng.standard_normal(shape)
+    bcs = (bc, m.PERIODIC_SOLVE, m.PERIODIC_SOLVE)
+
+    def view(off):
+        t = torch.full((f.size + 2,), -7.0, dtype=dt, device="cuda")
+        return t, t[off:off + f.size].view(shape)
+    for op in ("PADE6", "PENTA10", "COMPACT8", "COMPACT10", "TESTPADE"):
+        o = _make(op, 0, list(bcs), shape, prec)
+        if op.startswith("COMPACT"):
+            ref = O.filt(f, 0, op, G.OPS_ALPHA, bcs)
+        elif op == "TESTPADE":
+            ref = O.test_filter(f, 0, 1, bcs)
+        else:
+            ref = O.deriv(f, 0, op, bc, 1.0 / n if bc == m.PERIODIC_SOLVE else 1.0 / (n - 1.0))
+        for oi, oo in ((1, 0), (0, 1), (1, 1)):
+            x, (whole, y) = view(oi)[1], view(oo)
+            x.copy_(torch.tensor(f, dtype=dt))
+            (o.filterField if _is_filter(op) else o.calc1stDerivField)(x, y)
+            torch.cuda.synchronize()
+            assert H.rel_max(y.double().cpu().numpy(), ref) <= TOL[prec], (op, oi, oo)
+            edge = whole.cpu()
+            assert (edge[:oo] == -7.0).all() and (edge[oo + f.size:] == -7.0).all()
+
+
+@pytest.mark.parametrize("prec", [m.FP64, m.FP32BULK])
 def test_ragged_pass_through_lines(prec):
     """Filter lines on the faces of walls pass through in the ragged solve."""
     torch = _torch()
