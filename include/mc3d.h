@@ -147,7 +147,8 @@ typedef struct mc3d_config {
      * VREMAN (no averaging) or MLP (no DSM fallback: stages past
      * MLPFALLBACKFRAC are counted and keep the clamped network), no
      * sub-step filtering and no statistics. GPU.LEANSLAB (lean_slab):
-     * xi3-planes per slab (0: about 2^26 points). */
+     * xi3-planes per slab (0: about 2^26 points); up to three more where a
+     * slab would not end on a 16-byte boundary of the work fields. */
     int lean_storage;
     int lean_slab;
 } mc3d_config;

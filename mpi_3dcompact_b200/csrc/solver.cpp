@@ -1056,8 +1056,10 @@ int mc3d_solver_create(const mc3d_config *cfg, int device, mc3d_solver *out) {
         const long long plane = (long long)c.Nx * c.Ny;
         s->slab_nz = c.lean_slab > 0 ? std::min(c.lean_slab, c.Nz)
                                      : (int)std::max(1LL, std::min((long long)c.Nz, (1LL << 26) / plane));
-        // slabs start on an even point: the FP32 flux kernel loads and stores pairs
-        if (rb == sizeof(float) && plane % 2 && s->slab_nz % 2) s->slab_nz = std::min(s->slab_nz + 1, c.Nz);
+        // slabs start on a 16-byte boundary: the FP32 flux kernel loads and stores
+        // pairs, and the x sweeps' bulk copies need it (without it every other slab
+        // of an odd plane would go to another kernel, with another order of sums)
+        while ((long long)plane * s->slab_nz * rb % 16 && s->slab_nz < c.Nz) s->slab_nz++;
         const size_t ns = (size_t)plane * s->slab_nz;
         const bool two_n = c.rk_type == MC3D_KENRK4 || c.rk_type == MC3D_LSLDDRK4;
         for (int v = 0; v < 5 && !rc; v++) {

@@ -26,7 +26,8 @@ pytestmark = pytest.mark.gpu
 def _run(storage, prec, n_xyz, steps, ic, **kw):
     opts = dict(fd="PENTA10", filter="COMPACT8", alphaF=0.45, rk="LSLDDRK4", les="VREMAN", mu_ref=0.002, cfl=0.5)
     opts.update(kw)
-    s = m.CurvilinearCSolver(m.Options(grid=n_xyz, precision=prec, storage=storage, lean_slab=5, **opts))
+    opts.setdefault("lean_slab", 5)
+    s = m.CurvilinearCSolver(m.Options(grid=n_xyz, precision=prec, storage=storage, **opts))
     s.set_box_metrics(2 * math.pi)
     s.set_initial_conditions(*ic)
     s.step(steps)
@@ -65,10 +66,11 @@ def test_lean_fp32bulk_holds_the_fp64_bound():
 @pytest.mark.parametrize("prec,nx", [(m.FP64, 96), (m.FP64, 100), (m.FP64, 75), (m.FP32BULK, 75), (m.FP32BULK, 76),
                                      (m.FP32BULK, 128), (m.FP32BULK, 320)])
 def test_lean_accumulates_along_x(prec, nx):
-    """The lean dataflow's accumulating x sweep in each of its kernels: bulk-copied
-    tiles of whole segments and of ragged lines (one copy a tile, one a line, and
-    blocks that end inside 16 bytes), TMA-staged FP32 lines of two and five
-    segments. Bounds as above."""
+    """The lean dataflow's accumulating x sweep in each of its kernels: transposed
+    tiles of whole segments (FP64 96), bulk-copied tiles of ragged lines (one copy
+    a line: FP64 100; one a tile: 75, 76; with FP32 lines of 75 a last block that
+    ends inside 16 bytes), TMA-staged FP32 lines of two and five segments (128,
+    320). Bounds as above."""
     N = (nx, 25, 23)
     ic = [np.ascontiguousarray(a[:, :, :nx]) for a in _ic((nx + nx % 2, 25, 23), 11)]   # (an even box)
     q64, _ = _run("FULL", m.FP64, N, 4, ic)
@@ -78,6 +80,20 @@ def test_lean_accumulates_along_x(prec, nx):
             assert H.rel_max(q[i], q64[i]) <= 1e-12, (nx, i, H.rel_max(q[i], q64[i]))
         else:
             assert H.rel_l2(q[i], q64[i]) <= 1e-5, (nx, i, H.rel_l2(q[i], q64[i]))
+
+
+@pytest.mark.parametrize("prec", [m.FP64, m.FP32BULK])
+def test_lean_slabs_do_not_change_the_result(prec):
+    """Planes of 75 x 25 points, an odd number: slabs of five planes are enlarged
+    to end on a 16-byte boundary, so every slab takes the same kernels and the
+    state equals that of one slab over the block bit for bit."""
+    N = (75, 25, 23)
+    ic = [np.ascontiguousarray(a[:, :, :75]) for a in _ic((76, 25, 23), 11)]
+    qs, _ = _run("LEAN", prec, N, 4, ic)
+    q1, _ = _run("LEAN", prec, N, 4, ic, lean_slab=23)
+    for i in range(5):
+        assert np.isfinite(q1[i]).all()
+        assert np.array_equal(qs[i], q1[i]), (i, H.rel_max(qs[i], q1[i]))
 
 
 def test_lean_learned_closure_runs_and_counts_out_of_range_stages():
