@@ -314,6 +314,79 @@ def test_concurrent_solvers_on_own_streams_do_not_interfere():
     assert m.tma_wait_timeouts(0) == 0
 
 
+def _small_solver(N, prec, les):
+    """A block small enough that its gradient sweeps run on side streams."""
+    s = m.CurvilinearCSolver(m.Options(grid=N, fd="PENTA10", filter="COMPACT8", alphaF=0.45, mu_ref=1e-3,
+                                       rk="LSLDDRK4", les=les, les_avg="GLOBAL" if les == "DSM" else "NONE", cfl=0.5,
+                                       precision=prec))
+    s.set_box_metrics(2 * math.pi)
+    z, y, x = np.meshgrid(*[2 * math.pi * np.arange(n) / n for n in N[::-1]], indexing="ij")
+    s.set_initial_conditions(1.0 + 0.02 * np.cos(x + y), 0.3 * np.sin(x) * np.cos(y + z),
+                             0.2 * np.cos(2 * x - z) + 0.1 * np.sin(3 * y), 0.25 * np.sin(y) * np.cos(z),
+                             1.0 / 1.4 + 0.01 * np.sin(x - z))
+    return s
+
+
+@pytest.mark.parametrize("prec", [m.FP64, m.FP32BULK])
+@pytest.mark.parametrize("les", ["VREMAN", "DSM"])
+@pytest.mark.parametrize("N", [(64, 64, 64), (75, 49, 41)])
+def test_side_streams_do_not_change_the_step(N, les, prec):
+    """A timed solver runs every sweep on one stream, an untimed one runs the
+    gradient sweeps of a small block side by side (with DSM a second time, for
+    the corrected temperature): the same state bit for bit after three steps."""
+    q = []
+    for timing in (True, False):
+        s = _small_solver(N, prec, les)
+        s.set_timing(timing)
+        s.step(3)
+        q.append(s.conserved())
+    for i in range(5):
+        assert np.isfinite(q[0][i]).all()
+        assert np.array_equal(q[0][i], q[1][i]), i
+
+
+@pytest.mark.parametrize("les", ["VREMAN", "DSM"])
+def test_small_solvers_overlap_other_streams_work(les):
+    """Two small solvers with side streams, each on a stream of its own, and
+    operator calls on the legacy default stream, queued without waiting: in
+    each of five trials both states and the operator results equal their solo
+    runs bit for bit."""
+    import torch
+    cases = [((64, 64, 64), m.FP32BULK), ((75, 49, 41), m.FP64)]
+    ref = []
+    for N, prec in cases:
+        s = _small_solver(N, prec, les)
+        s.step(6)
+        ref.append(s.conserved())
+    g = torch.Generator(device="cuda").manual_seed(4)
+    xs = [torch.randn((64, 96, 75), device="cuda", generator=g, dtype=torch.float64) for _ in range(4)]
+    ops = [m.Penta10(xs[0].shape, m.PERIODIC_SOLVE, d) for d in range(3)]
+    solo = [[torch.empty_like(x) for x in xs] for _ in ops]
+    for op, ys in zip(ops, solo):
+        op.calc1stDerivFields(xs, ys)
+    torch.cuda.synchronize()
+    streams = [torch.cuda.Stream() for _ in cases]
+    for trial in range(5):
+        solvers = [_small_solver(N, prec, les) for N, prec in cases]
+        for s, st in zip(solvers, streams):
+            s.set_stream(st.cuda_stream)
+        outs = [[torch.zeros_like(x) for x in xs] for _ in ops]
+        torch.cuda.synchronize()
+        for _ in range(6):
+            for s in solvers:
+                s.step(1)
+            for op, ys in zip(ops, outs):
+                op.calc1stDerivFields(xs, ys)
+        got = [s.conserved() for s in solvers]
+        torch.cuda.synchronize()
+        for k in range(2):
+            for i in range(5):
+                assert np.array_equal(got[k][i], ref[k][i]), (trial, k, i)
+        for ys, rs in zip(outs, solo):
+            for y, r in zip(ys, rs):
+                assert torch.equal(y, r), trial
+
+
 def test_operator_calls_on_default_stream_overlap_a_solver_step():
     """Operator calls on the legacy default stream (mc3d_op_apply with a NULL
     stream, as a reference-side adapter makes them: FP32 Penta10 along x, y
