@@ -1,16 +1,19 @@
 // Register-resident segmented line solve.
 //
 // One CTA = S warps on a tile of W = 32 lines of one field; warp w owns rows
-// [w L, (w+1) L) of every line (L = N/S, a compile-time 32 or 64) and each
+// [w L, (w+1) L) of every line (L a compile-time 32 or 64, S = ceil(N/L); where
+// L does not divide N the last segment is completed by rows of zeros) and each
 // lane keeps its line's L rows, plus H halo rows on either side, in registers
 // for the whole solve:
 //   load      strided lines (y, z): one coalesced 128-byte row per warp load,
-//             straight into registers; x lines: the tile is staged transposed
-//             in shared memory once and each lane reads its line from there;
+//             straight into registers; x lines of whole segments: the tile is
+//             staged transposed in shared memory once and each lane reads its
+//             line from there; ragged x lines: the tile, contiguous in memory,
+//             comes by bulk copies and each lane reads its own line;
 //   pass 1    RHS stencil from registers and the forward elimination with a
 //             zero incoming state;
-//   chain     warp 0 chains the S segment end states (host-computed
-//             homogeneous responses at the segment ends);
+//   chain     each warp chains the end states of the segments before its own
+//             (host-computed homogeneous responses at the segment ends);
 //   fold      the incoming forward state is propagated through the segment's
 //             first rows by the elimination's own recurrence (no per-row
 //             response loads), while it is above the precision's cut-off;
@@ -690,10 +693,13 @@ __device__ __forceinline__ void rag_load_rows(int a, int N, const Row &row, R (&
 }
 
 // y and z lines whose length is no multiple of L (the RAG form of reg_solve):
-// S = ceil(N / L) warps, the last with the rows that are left. Bound by the
-// latency of the recurrences; the whole-line kernel that served such lengths
-// before kept one warp a tile busy with N-row recurrences through shared memory
-// (FP64 y derivatives of four 84 x 187 x 146 fields: 91 us there, 55 us here).
+// S = ceil(N / L) warps, the last with the rows that are left, against one warp a
+// tile and N-row recurrences through shared memory in the whole-line kernel (FP64
+// y derivatives of four 84 x 187 x 146 fields: 91 us there, 55 us here). Bound by
+// latency: 128 registers a thread leave 14 to 16 warps an SM, which issue in a
+// third of the cycles and wait on their own dependences, loads and the two
+// barriers (y and z derivatives of four 300 x 194 x 150 FP64 fields 169 and 166 us,
+// 3.3 TB/s).
 template <int DIR, typename R, int KIND, int H, int L, int E>
 __global__ void __launch_bounds__(512) sweep_rag_kernel(Grid3 g, LineOpDev<R> op, SweepBatch<R> b,
                                                         RhsFinalArgs<R> rf, int pass_y, int pass_z, int pass_x) {
@@ -747,11 +753,11 @@ static __device__ int g_bulk_wait_timeouts;
 // tile's pitch differs), read and overwritten by each lane along its own line,
 // and stored by bulk copies: no instruction per element but the lane's own
 // shared loads and stores. The accumulating sweep's operand takes the tile
-// while the lanes solve. Against a transposed tile filled by one cp.async per
-// element: three-direction gradients of four FP64 fields of 150 x 97 x 75 107 us
-// / 97 us, channel step of 100 x 97 x 60 907 us / 871 us. Lines of whole segments
-// keep the transposed tile: their even pitches make four lanes share a bank
-// (64^3 FP64 step 410 us there, 442 us here).
+// while the lanes solve. Lines of whole segments keep sweep_reg_kernel's transposed
+// tile: their even pitches put four lanes in a bank here. Bound by latency as the y
+// and z form is (x derivatives of four FP64 fields: 150 x 97 x 75 points at 15 warps
+// an SM; 300 x 194 x 150 at one CTA of 10 warps, 275 us, 2.0 TB/s, most of it
+// waiting at the barriers and on the recurrences).
 template <typename R, int KIND, int H, int L, int E>
 __global__ void __launch_bounds__(512) sweep_rag_x_kernel(Grid3 g, LineOpDev<R> op, SweepBatch<R> b, int pass_y,
                                                       int pass_z) {

@@ -373,10 +373,11 @@ __device__ __forceinline__ void tma_x_rows(const unsigned char *tile, int lane, 
 // x lines too long for the persistent kernel's two tiles, and the accumulating
 // sweep: one CTA per tile and one tile, which takes the previous output (the
 // accumulate's operand) while the lanes solve and then the results, which leave
-// by TMA store. Against the register kernel this replaces one asynchronous copy,
-// one transposed shared store and load and one global store per element with
-// bulk copies and 16-byte shared accesses (COMPACT10 of five 512 x 256 x 64
-// fields in three directions: 319 us there, 300 us here).
+// by TMA store: bulk copies and 16-byte shared accesses where the register kernel
+// has one asynchronous copy, a transposed shared store and load and one global
+// store per element (COMPACT10 of five 512 x 256 x 64 fields in three directions:
+// 319 us there, 300 us here). Bound by latency at two CTAs (16 warps) an SM, which
+// issue in 44% of the cycles: 106 us for those fields' x sweep, 3.2 TB/s.
 template <int KIND, int H, int L, int E>
 __global__ void __launch_bounds__(512) sweep_tma_x_kernel(Grid3 g, LineOpDev<float> op,
                                                           const __grid_constant__ TmaMaps maps, int pass_y,

@@ -204,6 +204,8 @@ int launch_sweep_tma_x(const Grid3 &g, const LineOpDev<float> &op, const SweepBa
     // lines in 64-row segments (up to 1024 values: 16 segments)
     if (!(epi == EPI_STORE || ((epi == EPI_STORE_NEG || epi == EPI_SUB) && !px && !py && !pz))) return MC3D_ERR_CONFIG;
     if (op.L != 64 || op.N % TMA_BOX != 0 || op.N > 1024 || op.N != g.Nx) return MC3D_ERR_CONFIG;
+    // (where the order of sums is kept: plain stores give the register kernel's bits at
+    // every length, the negated and accumulating sweeps do not)
     if (op.keep && (op.N > 256 || epi == EPI_SUB || b.nf > TMA_MAXF)) return MC3D_ERR_CONFIG;
     // one launch per TMA_MAXF fields. Every launch's maps are made before the
     // first launch: nothing has run yet when the batch turns out not to be covered
