@@ -559,7 +559,7 @@ LineSegments responses(const LineOpHost &h, int S, int L, int precision) {
 // shared-memory kernel, and, where the register kernel's length does not divide
 // N, its ragged ones as well (calls that form does not take, such as x lines off
 // a 16-byte boundary, use the equal ones).
-void segment(LineOpHost &h, int precision, bool ragged) {
+void segment(LineOpHost &h, int precision) {
     const int n = h.N;
     h.seg = LineSegments();
     h.rseg = LineSegments();
@@ -583,8 +583,7 @@ void segment(LineOpHost &h, int precision, bool ragged) {
             h.seg = responses(h, S, n / S, precision);
             break;
         }
-    if (!ragged || (precision != MC3D_FP64 && h.H <= 3 && !antisymmetric(h)))   // (the FP32 solve of H <= 3: derivatives only)
-        return;
+    if (precision != MC3D_FP64 && h.H <= 3 && !antisymmetric(h)) return;   // (the FP32 solve of H <= 3: derivatives only)
     if (int Lg = ragged_segment_len(n, h.kind)) {
         h.L = Lg;
         h.rag = true;
@@ -651,7 +650,7 @@ void fill_dev(const LineOpHost &h, const char *base, const Layout &lo, LineOpDev
     d.sbb = h.seg.S > 1 ? sg + 3 * n : nullptr;
     d.L = h.L;
     d.rag = h.rag;
-    d.keep = h.keep;
+    d.keep = 0;
     d.pf = h.L ? p + lo.pf : nullptr;
     d.pb = h.L ? p + lo.pb : nullptr;
     d.pz = h.L && h.kind == K_PEN_PER ? p + lo.pz : nullptr;
@@ -773,12 +772,11 @@ int ragged_segment_len(int N, int kind) {
     return 32;
 }
 
-int upload_line_op(const LineOpHost &hin, int precision, LineOpBuf &out, bool ragged) {
+int upload_line_op(const LineOpHost &hin, int precision, LineOpBuf &out) {
     LineOpHost h = hin;
     if (h.bw > MC3D_BWMAX) return fail(MC3D_ERR_CONFIG, "boundary row wider than the kernels support");
     analyse(h, precision);
-    segment(h, precision, ragged);
-    h.keep = !ragged;
+    segment(h, precision);
     out.precision = precision;
     MC3D_CUDA_TRY(cudaGetDevice(&out.device));
     Layout lo;

@@ -110,7 +110,6 @@ struct LineOpHost {
     LineSegments seg, rseg;
     int L = 0;   // segment length of the register-resident kernel (0: not used)
     bool rag = false;   // N is no multiple of L: the last segment (of rseg) has fewer rows
-    bool keep = false;  // uploaded without `ragged`: keep the order (and contraction) of the sums
 };
 
 // Segment length of the register-resident line solve for a line of N points
@@ -158,7 +157,7 @@ struct LineOpDev {
     //   phi[0..BWMAX-1], tail right-aligned on phi[N-BWMAX..N-1])
     int L;
     int rag;   // N is no multiple of L: the last of ceil(N / L) segments has fewer rows
-    int keep;  // long FP32 x lines stay with the register kernel (upload_line_op without `ragged`)
+    int keep;  // long FP32 x lines stay with the register kernel (whole_line_order)
     const R *pf, *pb, *pz, *sf2, *sb2, *hp, *tp;
     // FP32 derivative form of the register-resident solve (H <= 3): asym is 1
     // when the interior stencil is antisymmetric with a zero centre, sta[k-1]
@@ -180,9 +179,16 @@ struct LineOpBuf {
     int precision = MC3D_FP64;
     int device = 0;
 };
-// ragged: lines that are no multiple of the segment length may be solved in
-// segments, whose superposition sums in another order than the whole-line solve
-int upload_line_op(const LineOpHost &h, int precision, LineOpBuf &out, bool ragged = true);
+int upload_line_op(const LineOpHost &h, int precision, LineOpBuf &out);
+// The operator with one order of sums for every line length: equal segments or
+// the whole line where the ragged solve would take it, and the register kernel
+// for the long x lines.
+template <typename R>
+inline LineOpDev<R> whole_line_order(LineOpDev<R> d) {
+    d.keep = 1;
+    if (d.rag) d.L = d.rag = 0;
+    return d;
+}
 void free_line_op(LineOpBuf &b);
 
 // ---- sweep launch ---------------------------------------------------------

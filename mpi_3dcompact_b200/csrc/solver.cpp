@@ -54,6 +54,7 @@ struct mc3d_solver_s {
     mc3d_mlp mlp = nullptr;
     int *mlp_flag = nullptr, *mlp_flag_host = nullptr;
     long long mlp_fallbacks = 0;
+    bool whole_order = false;   // line solves keep the whole-line order of sums (dynamic_fp32)
     double *met64[10] = {};
     void *metR[10] = {};
     bool const_met = true;
@@ -106,18 +107,16 @@ struct mc3d_solver_s {
 
 namespace mc3d {
 
-// Whether a solver's (or SGS object's) lines may take the ragged segmented solve
-// and the long-line TMA kernels. Not in FP32 where the dynamic model can run:
-// its coefficient is a ratio of averages that magnifies the operators' rounding
-// (another order of the same FP32 sums moves the spanwise momentum of an O-grid
-// by 2e-5 relative within two steps, the distance of either from FP64 being
-// 4e-5), so every such run keeps one order of sums, the whole-line one: the DSM
-// solver, the standalone DSM object, and the learned closure's solver unless no
-// stage of it can fall back to DSM.
-static bool ragged_lines(const mc3d_config &c) {
-    const bool dynamic = c.les_model == MC3D_DSM ||
-                         (c.les_model == MC3D_MLPSGS && !c.lean_storage && c.mlp_fallback_frac < 1.0);
-    return !(dynamic && c.precision != MC3D_FP64);
+// Whether the dynamic model can run in FP32. Its coefficient is a ratio of averages
+// that magnifies the operators' rounding (another order of the same FP32 sums moves
+// the spanwise momentum of an O-grid by 2e-5 relative within two steps, the
+// distance of either from FP64 being 4e-5), so what it runs in keeps one order of
+// sums, the whole-line one (whole_line_order): every sweep of the DSM solver and of
+// the standalone DSM object, and of the learned closure's solver the stages that
+// fall back to DSM. Metrics are formed once, with that order wherever the model
+// can run.
+static bool dynamic_fp32(const mc3d_config &c) {
+    return c.precision != MC3D_FP64 && (c.les_model == MC3D_DSM || (c.les_model == MC3D_MLPSGS && !c.lean_storage));
 }
 
 // The dynamic model's test filter along d: DSMTESTFILTER 1 -> Pade, 2 -> explicit
@@ -127,7 +126,7 @@ static int upload_test_filter(mc3d_solver s, int d) {
     const int N[3] = {c.Nx, c.Ny, c.Nz};
     return upload_line_op(build_testfilter_op(c.dsm_test_filter == 1 ? MC3D_TESTFILTER_PADE : MC3D_TESTFILTER_EXP,
                                               c.bc_type[d], N[d]),
-                          c.precision, s->top[d], ragged_lines(c));
+                          c.precision, s->top[d]);
 }
 
 // Blocks up to this many points run their gradient sweeps side by side: faster at
@@ -251,7 +250,8 @@ static int sweep_on(mc3d_solver s, const Grid3 &g, int dir, const LineOpBuf &op,
     if (epi == EPI_RHS_FINAL) bytes = (3.0 * nf + (quirk ? 3.0 : 0.0)) * sizeof(R) * (double)g.n();
     int rc = tic(s, KC_SWEEP, bytes);
     if (rc) return rc;
-    rc = launch_sweep<R>(dir, g, opdev<R>(op), b, epi, rf, s->cfg.bc_type, filter, on ? *on : s->stream);
+    rc = launch_sweep<R>(dir, g, s->whole_order ? whole_line_order(opdev<R>(op)) : opdev<R>(op), b, epi, rf,
+                         s->cfg.bc_type, filter, on ? *on : s->stream);
     if (rc) return rc;
     return toc(s);
 }
@@ -578,6 +578,7 @@ template <typename R>
 static int stage_rhs(mc3d_solver s, double *const *qP) {
     int rc;
     bool dsm = s->cfg.les_model == MC3D_DSM;
+    if (s->cfg.les_model == MC3D_MLPSGS) s->whole_order = false;
     // gradients of U, V, W, T in each direction: der[3*var + dir]; with DSM
     // the T gradient waits for the tau_kk correction of T
     void *grad[3][4];
@@ -627,6 +628,12 @@ static int stage_rhs(mc3d_solver s, double *const *qP) {
         if ((double)*s->mlp_flag_host > s->cfg.mlp_fallback_frac * (double)s->g.n()) {
             s->mlp_fallbacks++;
             dsm = true;
+            // the rest of the stage in the dynamic model's order, the velocity
+            // gradients again where they came from the ragged solve
+            s->whole_order = dynamic_fp32(s->cfg);
+            if (s->whole_order && (s->dop[0].f32.rag || s->dop[1].f32.rag || s->dop[2].f32.rag) &&
+                (rc = gradients3<R>(s, 3, s->prim + 1, grad)))
+                return rc;
         } else {
             fp.les = 3;   // mu_sgs and k_sgs fields, no tau_kk
         }
@@ -1015,6 +1022,7 @@ int mc3d_solver_create(const mc3d_config *cfg, int device, mc3d_solver *out) {
     s->cfg = c;
     s->device = device;
     s->prec = c.precision;
+    s->whole_order = c.les_model == MC3D_DSM && dynamic_fp32(c);
     s->g = Grid3{c.Nx, c.Ny, c.Nz};
     s->host_time_step = c.time_step0;
     for (int f = 0; f < 6; f++) {
@@ -1047,9 +1055,9 @@ int mc3d_solver_create(const mc3d_config *cfg, int device, mc3d_solver *out) {
             LineOpHost dh = build_deriv_op(c.fd_type[d], c.bc_type[d], N[d], s->dxi[d]);
             LineOpHost fh = build_filter_op(c.filter_type, c.alphaF, c.bc_type[d], N[d]);
             LineOpHost vh = build_filter_op(MC3D_COMPACT10, -0.49, c.bc_type[d], N[d]);
-            if ((rc = upload_line_op(dh, c.precision, s->dop[d], ragged_lines(c)))) break;
-            if ((rc = upload_line_op(fh, c.precision, s->fop[d], ragged_lines(c)))) break;
-            if ((rc = upload_line_op(vh, c.precision, s->vop[d], ragged_lines(c)))) break;
+            if ((rc = upload_line_op(dh, c.precision, s->dop[d]))) break;
+            if ((rc = upload_line_op(fh, c.precision, s->fop[d]))) break;
+            if ((rc = upload_line_op(vh, c.precision, s->vop[d]))) break;
             if ((c.les_model == MC3D_DSM || c.les_model == MC3D_MLPSGS) && (rc = upload_test_filter(s, d))) break;
         }
     } catch (const std::exception &ex) {
@@ -1285,7 +1293,8 @@ static int metric_deriv(mc3d_solver s, int d, const MetricDir &md, const double 
     if (!tpb) {
         b.in[0] = in;
         b.out[0] = out;
-        return launch_sweep<double>(d, s->g, md.deriv.f64, b, EPI_STORE, rf, s->cfg.bc_type, false, s->stream);
+        return launch_sweep<double>(d, s->g, dynamic_fp32(s->cfg) ? whole_line_order(md.deriv.f64) : md.deriv.f64, b,
+                                    EPI_STORE, rf, s->cfg.bc_type, false, s->stream);
     }
     TpbArgs a{};
     a.N = d == 0 ? s->g.Nx : (d == 1 ? s->g.Ny : s->g.Nz);
@@ -1305,7 +1314,8 @@ static int metric_deriv(mc3d_solver s, int d, const MetricDir &md, const double 
     if (rc) return rc;
     b.in[0] = tmp;
     b.out[0] = out;
-    return launch_sweep<double>(d, s->g, md.solve.f64, b, EPI_STORE, rf, s->cfg.bc_type, false, s->stream);
+    return launch_sweep<double>(d, s->g, dynamic_fp32(s->cfg) ? whole_line_order(md.solve.f64) : md.solve.f64, b,
+                                EPI_STORE, rf, s->cfg.bc_type, false, s->stream);
 }
 
 // solveForJacobians (src/AbstractSingleBlockMesh.cpp:23-1308) on the device.
@@ -1349,7 +1359,7 @@ static int compute_metrics(mc3d_solver s, const double *hx, const double *hy, co
     try {
         for (int d = 0; d < 3 && !rc; d++) {
             LineOpHost h = build_deriv_op(s->cfg.fd_type[d], s->cfg.bc_type[d], Ns[d], s->dxi[d]);
-            if ((rc = upload_line_op(h, MC3D_FP64, md[d].deriv, ragged_lines(s->cfg)))) break;
+            if ((rc = upload_line_op(h, MC3D_FP64, md[d].deriv))) break;
             md[d].periodic = s->cfg.bc_type[d] == MC3D_PERIODIC_SOLVE;
             md[d].cd2 = s->cfg.fd_type[d] == MC3D_CD2;
             md[d].H = h.H;
@@ -1361,7 +1371,7 @@ static int compute_metrics(mc3d_solver s, const double *hx, const double *hy, co
                 sv.st[sv.H] = 1.0;
                 sv.deriv = false;
                 sv.inv_dh = 1.0;
-                rc = upload_line_op(sv, MC3D_FP64, md[d].solve, ragged_lines(s->cfg));
+                rc = upload_line_op(sv, MC3D_FP64, md[d].solve);
             }
         }
     } catch (const std::exception &e) {
@@ -2359,6 +2369,7 @@ int mc3d_sgs_create(int model, int averaging, int test_filter, int use_taukk, in
     for (int d = 0; d < 3; d++) s->cfg.bc_type[d] = bc_types[d];
     s->device = device;
     s->prec = precision;
+    s->whole_order = model == MC3D_DSM && dynamic_fp32(s->cfg);
     s->g = Grid3{Nx, Ny, Nz};
     for (int d = 0; d < 3; d++) s->dxi[d] = dxi[d];
     int rc = MC3D_OK;

@@ -340,29 +340,32 @@ def test_forced_fallback_equals_the_dsm_solver_on_ragged_lines():
     """FP32 on lines of 75, 34 and 40 points: a closure whose training range no
     state can lie in sends every stage to DSM, and the state after two steps
     equals a DSM solver's bit for bit (one order of the operators' sums wherever
-    the dynamic model can run, whose coefficient magnifies their rounding)."""
+    the dynamic model runs, whose coefficient magnifies their rounding). Without
+    a fallback the fallback fraction changes nothing."""
     N = (75, 34, 40)
     z, y, x = np.meshgrid(*[2 * math.pi * np.arange(n) / n for n in N[::-1]], indexing="ij")
     ic = [1.0 + 0.02 * np.cos(x + y), 0.3 * np.sin(x) * np.cos(y + z), 0.2 * np.cos(2 * x - z) + 0.1 * np.sin(3 * y),
           0.25 * np.sin(y) * np.cos(z) + 0.1 * np.cos(4 * x), 1.0 / 1.4 + 0.01 * np.sin(x - z)]
     net = m.MLPClosure(seed=6)
     one = np.ones(9, np.float32)
-    net.set_normalization(0 * one, one, 1e30 * one, 1e31 * one, np.zeros(2, np.float32), np.ones(2, np.float32))
     out = {}
-    for les in ("DSM", "MLP"):
+    for les, frac, lo in (("DSM", 1e-3, 0.0), ("MLP", 1e-3, 1e30), ("MLP", 1e-3, -1e31), ("MLP", 1.0, -1e31)):
+        net.set_normalization(0 * one, one, lo * one, 1e31 * one, np.zeros(2, np.float32), np.ones(2, np.float32))
         s = m.CurvilinearCSolver(m.Options(grid=N, fd="PADE6", filter="COMPACT10", alphaF=0.49, rk="RK4", mu_ref=1e-3,
-                                           les=les, les_avg="GLOBAL", precision=m.FP32BULK, mlp_fallback_frac=1e-3))
+                                           les=les, les_avg="GLOBAL", precision=m.FP32BULK, mlp_fallback_frac=frac))
         s.set_box_metrics(2.0 * math.pi)
         s.set_initial_conditions(*ic)
         if les == "MLP":
             s.set_mlp(net)
         s.step(2)
-        out[les] = s.conserved()
+        out[les, frac, lo] = s.conserved()
         if les == "MLP":
-            assert s.mlp_fallbacks() == 8
+            assert s.mlp_fallbacks() == (8 if lo > 0 else 0)
+    dsm, back, inside, clamped = out.values()
     for i in range(5):
-        assert np.isfinite(out["DSM"][i]).all()
-        assert np.array_equal(out["DSM"][i], out["MLP"][i]), (i, float(np.abs(out["DSM"][i] - out["MLP"][i]).max()))
+        assert np.isfinite(dsm[i]).all()
+        assert np.array_equal(dsm[i], back[i]), (i, float(np.abs(dsm[i] - back[i]).max()))
+        assert np.array_equal(inside[i], clamped[i]), i
 
 
 def test_standalone_dsm_object_keeps_the_solvers_order_of_sums():
