@@ -431,7 +431,7 @@ HBM_WORKLOAD = ("HBM-sizing: decaying HIT 1024^3 periodic box 2*pi, PENTA10, COM
 
 
 def hbm_sizing_run(args, local):
-    """the 1024^3 block held on one GPU by lean storage. The
+    """The 1024^3 block held on one GPU by lean storage. The
     initial field is made on the device (the reference generator's sequence,
     cuFFT), moved to host memory to free the device for the solver, and
     uploaded by set_initial_conditions. Device time of `steps` steps after

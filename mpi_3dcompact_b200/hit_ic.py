@@ -11,7 +11,7 @@ tests/hit/generate_init_hit.f90 (emathew1/MPI_3DCompact):
 The reference writes an ASCII Tecplot box of N+1 points; the solver grid is
 the periodic N^3 part of it, which is what this returns. Velocities are then
 scaled to a target turbulent Mach number (rms |u| / c, c = 1 for p = 1/gamma,
-rho = 1) as BASELINE's HIT configurations ask.
+rho = 1).
 """
 from __future__ import annotations
 

@@ -1,4 +1,4 @@
-"""Meshes of BASELINE's configurations (the role of the reference's
+"""Meshes of the supported flow configurations (the role of the reference's
 AbstractSingleBlockMesh::getMesh subclasses, e.g.
 src/AlgebraicSingleBlockMesh.hpp:210-266 for its cylinder), as (x, y, z)
 arrays shaped (Nz, Ny, Nx), x fastest, for CurvilinearCSolver.set_mesh."""

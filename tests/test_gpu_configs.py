@@ -1,9 +1,9 @@
-"""GPU checks of BASELINE's configurations against the reference solver run
+"""GPU checks of whole flow configurations against the reference solver run
 live on the same inputs: oracle/_ref/mc3d_ref, the reference's own C++
 compiled unchanged (it travels with the built library; these tests skip only
 where it was never built).
 
-* configs[0]: 64^3 HIT, PADE6 / RK4 / COMPACT10 alpha_f = 0.49, no SGS model,
+* 64^3 HIT, PADE6 / RK4 / COMPACT10 alpha_f = 0.49, no SGS model,
   CFL 0.5, Re_lambda about 30, FP64, 10 time steps: <= 1e-12 relative max error
   per conserved field, same time step count, time within 1e-12.
 * DSM with LESAVERAGING = LOCAL (src/AbstractSGS.cpp:149-160 through

@@ -217,7 +217,7 @@ def test_oracle_ten_steps_match_reference_fixture():
 
 @pytest.mark.skipif(not R.available(), reason="oracle/_ref/mc3d_ref not built")
 def test_reference_ogrid_dsm_local_nonfinite_at_128x64x32():
-    """The reference's own solver on BASELINE's O-grid configuration (cylinder,
+    """The reference's own solver on the O-grid configuration (cylinder,
     wall, cylindrical sponge, PADE6, KENRK4, COMPACT10, DSM with the Pade test
     filter and LOCAL averaging) at 128 x 64 x 32: after one time step the
     momentum and energy fields hold non-finite values (LOCAL divides by a
