@@ -435,7 +435,9 @@ int mc3d_solver_info(mc3d_solver s, int *time_step, double *time, double *dt, lo
  * (FP64 device reduction, synchronises). */
 int mc3d_solver_integrals(mc3d_solver s, double *kinetic, double *mass);
 
-/* The cudaStream_t the solver launches on (for event timing). By default every
+/* The cudaStream_t the solver launches on (for event timing; a block of up to
+ * 2^20 points also uses two streams of its own, forked from this one and joined
+ * to it again within each stage). By default every
  * solver on a device launches on one non-blocking stream of that device
  * (created at the first solver, kept until exit); mc3d_solver_set_stream
  * moves a solver to a stream of the caller's. */
